@@ -31,139 +31,257 @@ namespace ticc {
 
 constexpr int kPivotLd = kStride;  // the pivot block lives in a [128][kStride] shared tile
 constexpr int kSub = 64;           // Gauss-Jordan sub-block of the pivot block
-constexpr size_t kGJAuxDoubles = 2 * kSub + 4;  // Gauss-Jordan bookkeeping: pivot row, pivot column, candidates
-constexpr size_t kPivotAuxBytes = size_t(2) * kSub * kSub * sizeof(double) + kGJAuxDoubles * sizeof(double) + (4 + kSub) * sizeof(int);
+constexpr int kSmallLd = kSub + 4; // row stride of a 64-wide shared block: 4 mod 16, conflict-free DMMA fragments
+constexpr int kGJPanel = 8;        // columns of the sub-block that one warp owns and eliminates alone (one DMMA tile wide)
+constexpr size_t kGJAuxDoubles = kSub / kGJPanel + kSub;  // Gauss-Jordan bookkeeping: each panel's pivot rows as a mask; permutation and inverse
+constexpr size_t kPivotAuxBytes = (size_t(kSub) * kSmallLd + kGJAuxDoubles) * sizeof(double);
 constexpr size_t kPivotSmemBytes = size_t(kBlock) * kPivotLd * sizeof(double) + kPivotAuxBytes;
 constexpr size_t kUpdateSmemBytes = kUpdTileSmemBytes + 16;  // + the broadcast slot of the tile queue  // stages + C tile; the pivot aux reuses the stages
 static_assert(kPivotAuxBytes <= size_t(kUpdStageDoubles) * sizeof(double), "pivot scratch must fit in the update stages");
 
-// Gauss-Jordan exchange of a 64x64 sub-block S (row stride Ld) with partial
-// pivoting over its rows, by the kPivotThreads threads of the CTA; writes the inverse in
-// natural order to X (row stride kSub).  Thread t holds row t % 64, columns 16 (t / 64) ..
-// + 15 of the block in registers for the whole exchange: a step publishes only the pivot
-// row (its 4 owners) and the pivot column (one value per row) through shared memory, and the
-// next pivot is found as the maximum over the 32 rows of each of the 2 warps that
-// hold the next column (warp reductions on a rank key).  Pivot choice: largest magnitude among
-// the rows not yet used, the smallest row on ties, a NaN ranking as zero.  Two barriers per step.  Returns true if a
-// pivot was zero or non-finite.
-template <int Ld = kPivotLd>
-__device__ inline bool gauss_jordan_sub(double* S, double* X, double* aux) {
-  static_assert(kPivotThreads == 4 * kSub, "one thread per (row, 16-column group)");
-  double* prow = aux;
-  double* pcol = aux + kSub;
-  double* cand_val = aux + 2 * kSub;
-  int* cand_row = reinterpret_cast<int*>(cand_val + 4);
-  int* perm = cand_row + 4;
-  const int t = threadIdx.x, r = t & (kSub - 1), cg = t / kSub, lane = t & 31, half = r >> 5;
-  double v[16];
+// One warp's 8-column strip of a 64x64 block in DMMA accumulator layout: lane l holds row 8 mt + l / 4, columns
+// 2 (l % 4) and the next, for every 8-row tile mt.
+struct GJStrip {
+  double2 v[kSub / 8];
+};
+template <int Ld>
+__device__ __forceinline__ void gj_load_strip(GJStrip& g, const double* S, int c0) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = S[r * Ld + 16 * cg + i];
-  bool row_used = false, singular = false;
-  // this warp's best row for the next pivot to slot `half`.  Rank: 0 for a used row, else 1 +
-  // the bit pattern of the magnitude (a NaN as zero), which orders like the magnitude; the
-  // largest rank wins, the smallest row on ties: three warp reductions instead of shuffles.
-  unsigned long long* cand_key = reinterpret_cast<unsigned long long*>(cand_val);
-  auto candidate = [&](double m, bool excluded) {
-    const unsigned long long key = excluded ? 0ull : 1ull + (unsigned long long)__double_as_longlong(m >= 0.0 ? m : 0.0);
-    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-    const unsigned hmax = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned lmax = __reduce_max_sync(0xffffffffu, hi == hmax ? lo : 0u);
-    const unsigned rmin = __reduce_min_sync(0xffffffffu, (hi == hmax && lo == lmax) ? (unsigned)r : 0xffffffffu);
-    if (lane == 0) {
-      cand_key[half] = ((unsigned long long)hmax << 32) | lmax;
-      cand_row[half] = (int)rmin;
-    }
-  };
-  if (cg == 0) candidate(fabs(v[0]), false);
-  __syncthreads();
+  for (int mt = 0; mt < kSub / 8; ++mt) g.v[mt] = *reinterpret_cast<const double2*>(S + (8 * mt + (lane >> 2)) * Ld + c0 + 2 * (lane & 3));
+}
+template <int Ld>
+__device__ __forceinline__ void gj_store_strip(const GJStrip& g, double* S, int c0) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int mt = 0; mt < kSub / 8; ++mt) *reinterpret_cast<double2*>(S + (8 * mt + (lane >> 2)) * Ld + c0 + 2 * (lane & 3)) = g.v[mt];
+}
+
+// Panel update of a strip (columns c0 ..): new = (pivot row ? 0 : old) - E W with E the finished panel (columns j0 ..
+// j0 + 7 of S, all rows) and W the strip's old pivot rows, which pass through the strip's place in S.  No branch per row
+// (a divergent one costs some 50 cycles), and no full store of the strip (eight of them at once took the shared-memory
+// pipe 500 cycles): predicated stores.
+template <int Ld>
+__device__ __forceinline__ void gj_update_strip(GJStrip& g, double* S, const int* prow, int c0, int j0, unsigned long long rows_used) {
+  const int lane = threadIdx.x & 31, mr = lane >> 2, kr = lane & 3;
+  const unsigned lo = (unsigned)rows_used >> mr, hi = (unsigned)(rows_used >> 32) >> mr;
+  const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(S + mr * Ld + c0 + 2 * kr));
+#pragma unroll
+  for (int mt = 0; mt < kSub / 8; ++mt) {
+    const unsigned is_pivot = ((mt < 4 ? lo : hi) >> (8 * (mt & 3))) & 1u;
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.v2.f64 [%1], {%2, %3}; }" ::"r"(is_pivot), "r"(at + (unsigned)(8 * mt * Ld * sizeof(double))), "d"(g.v[mt].x), "d"(g.v[mt].y)
+                 : "memory");
+    g.v[mt].x = is_pivot ? 0.0 : g.v[mt].x;
+    g.v[mt].y = is_pivot ? 0.0 : g.v[mt].y;
+  }
+  __syncwarp();
+  const double w0 = -S[prow[kr] * Ld + c0 + mr], w1 = -S[prow[4 + kr] * Ld + c0 + mr];
+  const double* e = S + mr * Ld + j0 + kr;
+#pragma unroll
+  for (int mt = 0; mt < kSub / 8; ++mt) {
+    double acc[2] = {g.v[mt].x, g.v[mt].y};
+    dmma_8x8x4(acc, e[8 * mt * Ld], w0);
+    dmma_8x8x4(acc, e[8 * mt * Ld + 4], w1);
+    g.v[mt] = make_double2(acc[0], acc[1]);
+  }
+}
+
+// Eliminate the panel of columns j0 .. j0 + 7 of S by one warp (exchange steps inside the panel only).  Lane l holds
+// rows l and l + 32; rows in `rows_before` have been pivots (or do not take part).  Returns the panel's pivot rows as
+// a mask; prow[0..7] gets them in order.
+template <int Ld>
+__device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* prow, int j0, unsigned long long rows_before, bool& singular) {
+  const int lane = threadIdx.x & 31;
+  // rank of a row: its magnitude's leading 24 bits, then its index (the smaller row wins); 0 for a used row
+  constexpr unsigned kRankMask = ~127u;
+  unsigned mask0 = ((rows_before >> lane) & 1ull) ? 0u : kRankMask, mask1 = ((rows_before >> (lane + 32)) & 1ull) ? 0u : kRankMask;
+  unsigned code0 = mask0 ? 127u - lane : 0u, code1 = mask1 ? 95u - lane : 0u;
+  double v0[kGJPanel], v1[kGJPanel];
+#pragma unroll
+  for (int i = 0; i < kGJPanel; i += 2) {
+    const double2 x = *reinterpret_cast<const double2*>(S + lane * Ld + j0 + i), y = *reinterpret_cast<const double2*>(S + (lane + 32) * Ld + j0 + i);
+    v0[i] = x.x;
+    v0[i + 1] = x.y;
+    v1[i] = y.x;
+    v1[i + 1] = y.y;
+  }
+  // one column a turn, the registers rotating by one column, so that the body stays small: unrolled over a
+  // 16-column panel it was 50 KB of code and the fetch of its instructions took most of the time
 #pragma unroll 1
-  for (int blk = 0; blk < kSub / 16; ++blk) {
+  for (int jj = 0; jj < kGJPanel; ++jj) {
+    const unsigned h0 = (((unsigned)__double2hiint(v0[0]) << 1) & mask0) | code0, h1 = (((unsigned)__double2hiint(v1[0]) << 1) & mask1) | code1;
+    const bool second = h1 > h0;
+    const unsigned key = second ? h1 : h0;
+    const unsigned best = __reduce_max_sync(0xffffffffu, key);
+    constexpr unsigned kFirst = 1u << 21, kSpan = 0xffe00000u - kFirst;  // ranks of normal finite magnitudes
+    double c[kGJPanel];
 #pragma unroll
-    for (int jj = 0; jj < 16; ++jj) {
-      const int j = 16 * blk + jj;
-      const unsigned long long k0 = cand_key[0], k1 = cand_key[1];
-      int p = cand_row[0];
-      const int p1 = cand_row[1];
-      if (k1 > k0 || (k1 == k0 && p1 < p)) p = p1;
-      const bool mine = r == p;
-      if (mine) {
+    for (int i = 0; i < kGJPanel; ++i) c[i] = second ? v1[i] : v0[i];
+    const double inv_own = 1.0 / ((key - kFirst) < kSpan ? c[0] : 1.0);  // of every lane's candidate, beside the search
+    const int row = 127 - (int)(best & 127u);
+    const bool own0 = row == lane, own1 = row == lane + 32;
+    mask0 = own0 ? 0u : mask0;
+    code0 = own0 ? 0u : code0;
+    mask1 = own1 ? 0u : mask1;
+    code1 = own1 ? 0u : code1;
+    // the pivot row starts from zero with f = 1/a, every other row takes f = v/a
 #pragma unroll
-        for (int i = 0; i < 16; ++i) prow[16 * cg + i] = v[i];
-        row_used = true;
-      }
-      if (cg == blk) pcol[r] = v[jj];
-      if (t == 0) perm[j] = p;
-      __syncthreads();
-      double a = prow[j];
-      if (!(fabs(a) > 0.0) || !isfinite(a)) {
-        singular = true;
-        a = 1.0;
-      }
-      const double inv_a = 1.0 / a;
-      const double pc = pcol[r];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int c = 16 * cg + i;
-        const double pr = prow[c] * inv_a;
-        const double w = (c == j) ? pc * inv_a : v[i] - pc * pr;
-        v[i] = mine ? ((c == j) ? inv_a : -pr) : w;
-      }
-      if (j + 1 < kSub && cg == (j + 1) / 16) candidate(fabs(v[(jj + 1) & 15]), row_used);
-      __syncthreads();
+    for (int i = 1; i < kGJPanel; ++i) {
+      v0[i] = own0 ? 0.0 : v0[i];
+      v1[i] = own1 ? 0.0 : v1[i];
     }
+    v0[0] = own0 ? 1.0 : v0[0];
+    v1[0] = own1 ? 1.0 : v1[0];
+    singular |= !((best - kFirst) < kSpan);
+    if (lane == 0) prow[jj] = row;
+    const double inv = __shfl_sync(0xffffffffu, inv_own, row & 31);
+    double p[kGJPanel];
+#pragma unroll
+    for (int i = 1; i < kGJPanel; ++i) p[i] = __shfl_sync(0xffffffffu, c[i], row & 31);
+    const double f0 = v0[0] * inv, f1 = v1[0] * inv;
+#pragma unroll
+    for (int i = 0; i + 1 < kGJPanel; ++i) {
+      v0[i] = fma(-f0, p[i + 1], v0[i + 1]);
+      v1[i] = fma(-f1, p[i + 1], v1[i + 1]);
+    }
+    v0[kGJPanel - 1] = f0;
+    v1[kGJPanel - 1] = f1;
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) S[r * Ld + 16 * cg + i] = v[i];
-  __syncthreads();
+  for (int i = 0; i < kGJPanel; i += 2) {
+    *reinterpret_cast<double2*>(S + lane * Ld + j0 + i) = make_double2(v0[i], v0[i + 1]);
+    *reinterpret_cast<double2*>(S + (lane + 32) * Ld + j0 + i) = make_double2(v1[i], v1[i + 1]);
+  }
+  const unsigned long long all = ((unsigned long long)__ballot_sync(0xffffffffu, mask1 == 0u) << 32) | __ballot_sync(0xffffffffu, mask0 == 0u);
+  return all & ~rows_before;
+}
+
+// S <- S^{-1} (64x64 in shared memory, row stride Ld = 4 mod 16) by Gauss-Jordan exchange with partial pivoting over
+// the block's rows, by the kThreads threads of the CTA.  `n_act` (a multiple of kGJPanel): rows and columns at or beyond
+// it hold the identity and are left alone.  Returns true if a pivot was zero or non-finite.  Uses named barrier 1.
+//
+// The exchange of one column is a serial chain (rank the rows, reciprocal, publish the row, update), so the work around
+// that chain is what costs.  It is blocked: one warp eliminates a panel of 8 columns in registers, with no barrier, no
+// shared memory and no branch inside the chain (295 cycles a column, issue-bound; 200 in a panel of 4 and 370 in one of
+// 16, while the step from one panel to the next takes 800 at any width).  The other columns take the 8 exchanges as
+// one rank-8 product on the FP64 tensor pipe: each warp keeps the 8-column strips that it owns in accumulator
+// registers, so that a panel costs one CTA barrier.  The owner of the next panel updates its strip alone, then
+// eliminates while the others update theirs.
+// Pivot choice: the largest magnitude by its leading 24 bits (13 of mantissa) among the unused rows, the smallest row
+// on ties; a NaN or an infinity ranks above all and is reported, as is a zero (or subnormal) pivot.
+template <int Ld, int kThreads>
+__device__ inline bool gauss_jordan_sub(double* S, double* aux, int n_act = kSub) {
+  constexpr int kWarps = kThreads / 32, kOwn = kSub / kGJPanel / kWarps;
+  unsigned long long* panel_rows = reinterpret_cast<unsigned long long*>(aux);  // [kSub / kGJPanel]
+  int* perm = reinterpret_cast<int*>(aux + kSub / kGJPanel);
+  int* iperm = perm + kSub;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  bool singular = false;
+  const int panels = n_act / kGJPanel;
+  unsigned long long used = n_act == kSub ? 0ull : ~0ull << n_act;  // rows of all panels so far
+  GJStrip g[kOwn];
+#pragma unroll
+  for (int o = 0; o < kOwn; ++o) gj_load_strip<Ld>(g[o], S, kGJPanel * (warp + o * kWarps));
+  __syncwarp();
+#pragma unroll 1
+  for (int q = -1; q < panels; ++q) {
+    const int j0 = kGJPanel * q, next = q + 1;
+    unsigned long long mask = 0;
+    if (q >= 0) {
+      __syncthreads();  // panel q is in S; the updates of panel q - 1 are done
+      mask = panel_rows[q];
+      used |= mask;
+    }
+    const bool more = q + 1 < panels, mine = more && next % kWarps == warp;
+    if (mine) {  // the strip of the next panel first
+      if (q >= 0) {
+#pragma unroll
+        for (int o = 0; o < kOwn; ++o)
+          if (next == warp + o * kWarps) {
+            gj_update_strip<Ld>(g[o], S, perm + j0, kGJPanel * next, j0, mask);
+            gj_store_strip<Ld>(g[o], S, kGJPanel * next);
+          }
+        asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
+        __syncwarp();
+      }
+      const unsigned long long m = gj_factor_panel<Ld>(S, perm + j0 + kGJPanel, j0 + kGJPanel, used, singular);
+      if (lane == 0) panel_rows[q + 1] = m;
+    } else if (more && q >= 0) {
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");  // the next panel's owner has the tensor pipe to itself
+    }
+    if (q < 0) continue;
+#pragma unroll
+    for (int o = 0; o < kOwn; ++o) {
+      const int strip = warp + o * kWarps;
+      if (strip == q) gj_load_strip<Ld>(g[o], S, j0);
+      else if (strip < panels && !(mine && strip == next)) gj_update_strip<Ld>(g[o], S, perm + j0, kGJPanel * strip, j0, mask);
+    }
+  }
+  __syncthreads();  // the last panel's E has been read
+#pragma unroll
+  for (int o = 0; o < kOwn; ++o)
+    if (warp + o * kWarps < panels) gj_store_strip<Ld>(g[o], S, kGJPanel * (warp + o * kWarps));
   // inverse element (j, perm[c]) sits at exchange slot (perm[j], c)
-  int* iperm = reinterpret_cast<int*>(prow);
-  if (t < kSub) iperm[perm[t]] = t;
+  if (t < n_act) iperm[perm[t]] = t;
   __syncthreads();
-  for (int e = t; e < kSub * kSub; e += kPivotThreads) {
-    const int jj = e / kSub, m = e % kSub;
-    X[e] = S[perm[jj] * Ld + iperm[m]];
+  constexpr int kPer = kSub * kSub / kThreads;
+  double x[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int e = t + u * kThreads, j = e / kSub, m = e % kSub;
+    x[u] = (j < n_act && m < n_act) ? S[perm[j] * Ld + iperm[m]] : (j == m ? 1.0 : 0.0);
+  }
+  singular = __syncthreads_or(singular);
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int e = t + u * kThreads;
+    S[(e / kSub) * Ld + e % kSub] = x[u];
   }
   __syncthreads();
   return singular;
 }
 
-// C (64x64, row stride ldc) = sign * A (64x64, lda) * B (64x64, ldb) [+ C if accumulate];
-// 256 threads, 4x4 outputs each.  No aliasing between C and A/B.
+// C (64x64, row stride ldc) = sign * A (64x64, lda) * B (64x64, ldb) [+ C if accumulate] on the FP64 tensor
+// pipe; 256 threads, 16 x 32 outputs a warp, row strides 4 mod 16 (conflict-free fragments).  C may be B
+// or A: it is written after a barrier behind the last read.
 __device__ inline void small_gemm64(double* C, int ldc, const double* A, int lda, const double* B, int ldb, double sign, bool accumulate) {
-  const int t = threadIdx.x;
-  const int i0 = (t >> 4) * 4, m0 = (t & 15) * 4;
-  double acc[4][4] = {};
-  for (int k = 0; k < kSub; ++k) {
-    double a[4], b[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mr = lane >> 2, kr = lane & 3;
+  const int m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
+  double acc[2][4][2] = {};
+#pragma unroll 4
+  for (int k = 0; k < kSub; k += 4) {
+    double a[2], b[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = A[(i0 + u) * lda + k];
+    for (int u = 0; u < 2; ++u) a[u] = A[(m0 + 8 * u + mr) * lda + k + kr];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) b[u] = B[k * ldb + m0 + u];
+    for (int w = 0; w < 4; ++w) b[w] = B[(k + kr) * ldb + n0 + 8 * w + mr];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int w = 0; w < 4; ++w) acc[u][w] = fma(a[u], b[w], acc[u][w]);
+      for (int w = 0; w < 4; ++w) dmma_8x8x4(acc[u][w], a[u], b[w]);
   }
   __syncthreads();
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < 2; ++u)
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      double* d = C + (i0 + u) * ldc + m0 + w;
-      *d = accumulate ? *d + sign * acc[u][w] : sign * acc[u][w];
+      double2* d = reinterpret_cast<double2*>(C + (m0 + 8 * u + mr) * ldc + n0 + 8 * w + 2 * kr);
+      double2 c = accumulate ? *d : make_double2(0.0, 0.0);
+      c.x += sign * acc[u][w][0];
+      c.y += sign * acc[u][w][1];
+      *d = c;
     }
   __syncthreads();
 }
 
 // Sweep the 128x128 block held in shared memory (row stride kPivotLd) in place:
 // P <- -P^{-1}, through its two 64-wide sub-blocks (the same principal pivot transform
-// as the outer sweep, one level down).  aux holds two 64x64 temporaries and the
+// as the outer sweep, one level down).  aux holds a 64 x kSmallLd temporary and the
 // Gauss-Jordan bookkeeping.
 template <bool kSym>
 __device__ inline bool sweep_block(double* P, double* aux) {
-  double* X = aux;
-  double* U = aux + kSub * kSub;
-  double* gj = aux + 2 * kSub * kSub;
+  double* U = aux;
+  double* gj = aux + kSub * kSmallLd;
   bool singular = false;
   for (int s = 0; s < 2; ++s) {
     const int k0 = kSub * s, r0 = kSub * (1 - s);
@@ -171,24 +289,17 @@ __device__ inline bool sweep_block(double* P, double* aux) {
     double* Pkr = P + k0 * kPivotLd + r0;
     double* Prk = P + r0 * kPivotLd + k0;
     double* Prr = P + r0 * kPivotLd + r0;
-    singular |= gauss_jordan_sub(Pkk, X, gj);
-    small_gemm64(U, kSub, X, kSub, Pkr, kPivotLd, 1.0, false);     // U = P_KK^-1 P_KR
-    small_gemm64(Prr, kPivotLd, Prk, kPivotLd, U, kSub, -1.0, true);  // P_RR -= P_RK U
-    if (kSym) {
-      for (int e = threadIdx.x; e < kSub * kSub; e += kPivotThreads) {
-        const int i = e / kSub, m = e % kSub;
-        Pkr[i * kPivotLd + m] = U[e];
-        Prk[m * kPivotLd + i] = U[e];
-      }
-      __syncthreads();
-    } else {
-      for (int e = threadIdx.x; e < kSub * kSub; e += kPivotThreads) Pkr[(e / kSub) * kPivotLd + e % kSub] = U[e];
-      __syncthreads();
-      small_gemm64(U, kSub, Prk, kPivotLd, X, kSub, 1.0, false);     // V = P_RK P_KK^-1
-      for (int e = threadIdx.x; e < kSub * kSub; e += kPivotThreads) Prk[(e / kSub) * kPivotLd + e % kSub] = U[e];
-      __syncthreads();
+    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj);
+    small_gemm64(U, kSmallLd, Pkk, kPivotLd, Pkr, kPivotLd, 1.0, false);     // U = P_KK^-1 P_KR
+    small_gemm64(Prr, kPivotLd, Prk, kPivotLd, U, kSmallLd, -1.0, true);  // P_RR -= P_RK U
+    if (!kSym) small_gemm64(Prk, kPivotLd, Prk, kPivotLd, Pkk, kPivotLd, 1.0, false);  // V = P_RK P_KK^-1
+    for (int e = threadIdx.x; e < kSub * kSub; e += kPivotThreads) {
+      const int i = e / kSub, m = e % kSub;
+      const double u = U[i * kSmallLd + m];
+      Pkr[i * kPivotLd + m] = u;
+      Pkk[i * kPivotLd + m] = -Pkk[i * kPivotLd + m];
+      if (kSym) Prk[i * kPivotLd + m] = U[m * kSmallLd + i];
     }
-    for (int e = threadIdx.x; e < kSub * kSub; e += kPivotThreads) Pkk[(e / kSub) * kPivotLd + e % kSub] = -X[e];
     __syncthreads();
   }
   return singular;
@@ -253,34 +364,29 @@ __global__ void __launch_bounds__(kPivotThreads) sweep_pivot_kernel(double* __re
 
 // Sweep of a single-block matrix whose channels fill at most the leading 64 rows and
 // columns (the rest is identity padding): only the 64x64 block is inverted, in a CTA with
-// 69 KB of shared memory so that three matrices share an SM; the padding becomes -I.
-constexpr int kSmallLd = kSub + 4;
-constexpr size_t kPivot64SmemBytes = (size_t(kSub) * kSmallLd + size_t(kSub) * kSub + kGJAuxDoubles) * sizeof(double) + (4 + kSub) * sizeof(int);
+// 36 KB of shared memory so that several matrices share an SM; the padding becomes -I.
+constexpr size_t kPivot64SmemBytes = (size_t(kSub) * kSmallLd + kGJAuxDoubles) * sizeof(double);
 template <bool kSym>
-__global__ void __launch_bounds__(kPivotThreads) sweep_pivot64_kernel(double* __restrict__ M, long long mstride, int ld, int* status) {
+__global__ void __launch_bounds__(kPivotThreads) sweep_pivot64_kernel(double* __restrict__ M, long long mstride, int ld, int n_act, int* status) {
   extern __shared__ double smem[];
   double* S = smem;
-  double* X = S + kSub * kSmallLd;
-  double* gj = X + kSub * kSub;
+  double* gj = S + kSub * kSmallLd;
   const int b = blockIdx.x;
   double* Mb = M + (long long)b * mstride;
 #pragma unroll
   for (int u = 0; u < kSub * kSub / 2 / kPivotThreads; ++u) {
     const int piece = u * kPivotThreads + threadIdx.x;
-    const double2 m = *reinterpret_cast<const double2*>(Mb + (long long)(piece >> 5) * ld + (piece & 31) * 2);
-    double* d = S + (piece >> 5) * kSmallLd + (piece & 31) * 2;
-    d[0] = m.x;
-    d[1] = m.y;
+    *reinterpret_cast<double2*>(S + (piece >> 5) * kSmallLd + (piece & 31) * 2) = *reinterpret_cast<const double2*>(Mb + (long long)(piece >> 5) * ld + (piece & 31) * 2);
   }
   __syncthreads();
-  const bool singular = gauss_jordan_sub<kSmallLd>(S, X, gj);
+  const bool singular = gauss_jordan_sub<kSmallLd, kPivotThreads>(S, gj, n_act);
   if (singular && threadIdx.x == 0) report_status(status, kDeviceSingularPivot, b, 0);
   for (int idx = threadIdx.x; idx < ld * ld; idx += kPivotThreads) {
     const int i = idx / ld, j = idx % ld;
     double x;
     if (i < kSub && j < kSub) {
-      x = X[i * kSub + j];
-      if (kSym) x = 0.5 * (x + X[j * kSub + i]);
+      x = S[i * kSmallLd + j];
+      if (kSym) x = 0.5 * (x + S[j * kSmallLd + i]);
       x = -x;
     } else {
       x = (i == j) ? -1.0 : 0.0;
@@ -1241,7 +1347,7 @@ inline cudaError_t sweep_batched(double* M, long long mstride, int np, int batch
   if (e != cudaSuccess) return e;
   const int nt = np / kBlock;
   if (nt == 1 && n_used > 0 && n_used <= kSub) {
-    sweep_pivot64_kernel<kSym><<<batch, kPivotThreads, kPivot64SmemBytes, stream>>>(M, mstride, np, status);
+    sweep_pivot64_kernel<kSym><<<batch, kPivotThreads, kPivot64SmemBytes, stream>>>(M, mstride, np, (int)round_up(n_used, kGJPanel), status);
     note_launch();
     return cudaGetLastError();
   }
