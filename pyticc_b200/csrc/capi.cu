@@ -17,6 +17,7 @@
 #include "match.cuh"
 #include "pes.cuh"
 #include "sweep.cuh"
+#include "sweep_fine.cuh"
 #include "tc_update.cuh"
 
 namespace {
@@ -67,6 +68,13 @@ size_t ldmd_layout(ticc::LdmdLayout& L, int n, int n_energy, int n_block, int n_
   const size_t need_s = ticc::sweep_scratch_doubles(L.npr) * (size_t)(n_sector < 8 ? n_sector : 8);
   L.scratch_doubles = need_e > need_s ? need_e : need_s;
   L.scratch = c.take<double>(L.scratch_doubles);
+  const int used = is_complex ? 2 * n : n;
+  const size_t q_chunk = std::min((size_t)n_sector * n_block, L.scratch_doubles / ticc::sweep_scratch_doubles(L.npr));
+  const bool fine_m = precision == TICC_PRECISION_FP64 && ticc::use_fine(used, batch), fine_q = ticc::use_fine(n, q_chunk);
+  const size_t fine = std::max(fine_m ? ticc::fine_total_doubles(ticc::fine_tiles(used), batch) : 0, fine_q ? ticc::fine_total_doubles(ticc::fine_tiles(n), q_chunk) : 0);
+  double* fine_base = fine > 0 ? c.take<double>(fine) : nullptr;
+  L.fine = fine_m ? fine_base : nullptr;
+  L.fine_q = fine_q ? fine_base : nullptr;
   L.reduced = (precision == TICC_PRECISION_MIXED) ? c.take<int>((size_t)n_sector) : nullptr;
   L.split = (precision == TICC_PRECISION_MIXED) ? c.take<float>(ticc::tc_split_floats(L.np, (int)batch)) : nullptr;
   if (base == nullptr) L.reduced = nullptr, L.split = nullptr;
@@ -93,6 +101,8 @@ size_t match_layout(ticc::MatchLayout& L, int n, int n_energy, int is_complex, i
   L.C = c.take<double>((size_t)n_energy * L.npa * L.npa);
   const int np = L.npz > L.npa ? L.npz : L.npa;
   L.scratch = c.take<double>((size_t)n_energy * ticc::sweep_scratch_doubles(np));
+  const int used = is_complex ? 2 * n : n;
+  L.fine = ticc::use_fine(used, n_energy) ? c.take<double>(ticc::fine_total_doubles(ticc::fine_tiles(used), n_energy)) : nullptr;
   return c.used + 256;
 }
 
@@ -114,18 +124,20 @@ int ticc_last_error(char* buf, size_t len) {
 }
 
 // ---- symmetric inversion ---------------------------------------------------------------
-static size_t sym_layout(int n, int batch, int is_complex, double** M, double** scratch, char* base) {
+static size_t sym_layout(int n, int batch, int is_complex, double** M, double** scratch, char* base, double** fine = nullptr) {
   Carver c{base};
   const int np = ticc::ldmd_np(n, is_complex);
   *M = c.take<double>((size_t)batch * np * np);
   *scratch = c.take<double>((size_t)batch * ticc::sweep_scratch_doubles(np));
+  const int used = is_complex ? 2 * n : n;
+  if (fine != nullptr) *fine = ticc::use_fine(used, batch) ? c.take<double>(ticc::fine_total_doubles(ticc::fine_tiles(used), batch)) : nullptr;
   return c.used + 256;
 }
 
 int ticc_sym_inverse_workspace_size(int n, int batch, int is_complex, size_t* bytes) {
   if (n < 1 || batch < 1 || bytes == nullptr) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_sym_inverse_workspace_size: n=%d batch=%d", n, batch);
-  double *M, *s;
-  *bytes = sym_layout(n, batch, is_complex, &M, &s, nullptr);
+  double *M, *s, *fine;
+  *bytes = sym_layout(n, batch, is_complex, &M, &s, nullptr, &fine);
   return TICC_OK;
 }
 
@@ -175,16 +187,17 @@ __global__ void sym_store_kernel(const double* M, int np, double* dst, int n, in
 
 int ticc_sym_inverse(void* M, int n, int batch, int is_complex, void* workspace, size_t workspace_bytes, int* device_status, void* stream) {
   if (M == nullptr || n < 1 || batch < 1) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_sym_inverse: M=%p n=%d batch=%d", M, n, batch);
-  double *Mw, *scratch;
-  const size_t need = sym_layout(n, batch, is_complex, &Mw, &scratch, nullptr);
+  double *Mw, *scratch, *fine;
+  const size_t need = sym_layout(n, batch, is_complex, &Mw, &scratch, nullptr, &fine);
   if (workspace == nullptr || workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "ticc_sym_inverse: workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-  sym_layout(n, batch, is_complex, &Mw, &scratch, static_cast<char*>(workspace));
+  sym_layout(n, batch, is_complex, &Mw, &scratch, static_cast<char*>(workspace), &fine);
+  ticc::FineState state{fine};
   const int np = ticc::ldmd_np(n, is_complex);
   const long long nl = is_complex ? np / 2 : np;
   cudaStream_t s = as_stream(stream);
   sym_load_kernel<<<dim3(ticc::grid_for(nl * nl, 256, 8192), batch), 256, 0, s>>>(static_cast<double*>(M), n, is_complex, Mw, np);
   ticc::note_launch();
-  cudaError_t e = ticc::sweep_sym(Mw, (long long)np * np, np, batch, scratch, device_status, s, nullptr, is_complex ? 2 * n : n);
+  cudaError_t e = ticc::sweep_any(state, Mw, (long long)np * np, np, batch, scratch, device_status, s, nullptr, is_complex ? 2 * n : n, nullptr);
   if (e != cudaSuccess) return cuda_fail(e, "ticc_sym_inverse");
   sym_store_kernel<<<dim3(ticc::grid_for((long long)n * n, 256, 8192), batch), 256, 0, s>>>(Mw, np, static_cast<double*>(M), n, is_complex);
   ticc::note_launch();

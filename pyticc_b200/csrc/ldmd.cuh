@@ -16,7 +16,7 @@
 // energy-shared matrix per (sector, block).
 #pragma once
 
-#include "sweep.cuh"
+#include "sweep_fine.cuh"
 #include "ticc_common.cuh"
 
 namespace ticc {
@@ -45,6 +45,8 @@ struct LdmdLayout {
   double* scratch;
   size_t scratch_doubles;
   int* reduced;   // [n_sector] leading sweep blocks taken in TF32x3 (mixed mode), else null
+  double* fine;   // 64-tile sweeps' panels and flags (FP64 work matrices where they fit), else null
+  double* fine_q; // the same region for the Q_mid sweeps, else null
   float* split;   // FP32 operand panels of the reduced steps' tcgen05 update (mixed mode), else null
 };
 
@@ -398,9 +400,10 @@ inline cudaError_t ldmd_qmid(const LdmdSectors& sec, LdmdLayout& L, int* status,
   ldmd_qmid_build_kernel<<<dim3(grid_for(per, 256, 4096), count), 256, 0, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm);
   note_launch();
   const int chunk = (int)(L.scratch_doubles / sweep_scratch_doubles(L.npr));
+  FineState fine{L.fine_q};
   for (int s0 = 0; s0 < count; s0 += chunk) {
     const int cnt = (count - s0 < chunk) ? count - s0 : chunk;
-    cudaError_t e = sweep_sym(L.Qm + (long long)s0 * per, per, L.npr, cnt, L.scratch, status, stream, nullptr, L.n);
+    cudaError_t e = sweep_any(fine, L.Qm + (long long)s0 * per, per, L.npr, cnt, L.scratch, status, stream, nullptr, L.n, nullptr);
     if (e != cudaSuccess) return e;
   }
   ldmd_qmid_finish_kernel<<<dim3(grid_for(per, 256, 4096), count), 256, 0, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm);
@@ -425,14 +428,15 @@ inline cudaError_t ldmd_propagate(double* Y, const double* energies, double mu, 
   const dim3 grid((unsigned)nl, L.n_block);
   const long long mstride = (long long)L.np * L.np;
   const int used = L.is_complex ? 2 * L.n : L.n;  // rows of the work matrix beyond these are identity padding
+  FineState fine{L.fine};
   for (int s = 0; s < sec.n_sector; ++s) {
     ldmd_elementwise_kernel<<<grid, 256, 0, stream>>>(s == 0 ? 0 : 1, s, sec, L, Y, Y);
     note_launch();
-    err = sweep_sym(L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
+    err = sweep_any(fine, L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
     if (err != cudaSuccess) return err;
     ldmd_elementwise_kernel<<<grid, 256, 0, stream>>>(2, s, sec, L, Y, Y);
     note_launch();
-    err = sweep_sym(L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
+    err = sweep_any(fine, L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
     if (err != cudaSuccess) return err;
   }
   ldmd_elementwise_kernel<<<grid, 256, 0, stream>>>(3, sec.n_sector - 1, sec, L, Y, Y);

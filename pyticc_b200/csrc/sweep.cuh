@@ -86,6 +86,16 @@ __device__ __forceinline__ void gj_update_strip(GJStrip& g, double* S, const int
   }
 }
 
+// 1/a for a normal a (subnormal results flush to zero): the hardware's approximation y (relative error 2^-23) and one step of the
+// third-order Newton (Householder) iteration y (1 + e + e^2), e = 1 - a y, whose own error is e^3.  Four instructions
+// and no branch, so that the search around it can be scheduled into its latency (the divide operator ends a basic block).
+__device__ __forceinline__ double gj_reciprocal(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 // Eliminate the panel of columns j0 .. j0 + 7 of S by one warp (exchange steps inside the panel only).  Lane l holds
 // rows l and l + 32; rows in `rows_before` have been pivots (or do not take part).  Returns the panel's pivot rows as
 // a mask; prow[0..7] gets them in order.
@@ -117,7 +127,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
     double c[kGJPanel];
 #pragma unroll
     for (int i = 0; i < kGJPanel; ++i) c[i] = second ? v1[i] : v0[i];
-    const double inv_own = 1.0 / ((key - kFirst) < kSpan ? c[0] : 1.0);  // of every lane's candidate, beside the search
+    const double inv_own = gj_reciprocal((key - kFirst) < kSpan ? c[0] : 1.0);  // of every lane's candidate, beside the search
     const int row = 127 - (int)(best & 127u);
     const bool own0 = row == lane, own1 = row == lane + 32;
     mask0 = own0 ? 0u : mask0;
@@ -169,8 +179,13 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
 // eliminates while the others update theirs.
 // Pivot choice: the largest magnitude by its leading 24 bits (13 of mantissa) among the unused rows, the smallest row
 // on ties; a NaN or an infinity ranks above all and is reported, as is a zero (or subnormal) pivot.
+// gauss_jordan_exchange leaves S in exchange form: inverse element (j, m) is S[perm[j] * Ld + iperm[m]] (j, m < n_act).
+struct GJOrder {
+  const int* perm;
+  const int* iperm;
+};
 template <int Ld, int kThreads>
-__device__ inline bool gauss_jordan_sub(double* S, double* aux, int n_act = kSub) {
+__device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& order, int n_act = kSub) {
   constexpr int kWarps = kThreads / 32, kOwn = kSub / kGJPanel / kWarps;
   unsigned long long* panel_rows = reinterpret_cast<unsigned long long*>(aux);  // [kSub / kGJPanel]
   int* perm = reinterpret_cast<int*>(aux + kSub / kGJPanel);
@@ -221,20 +236,26 @@ __device__ inline bool gauss_jordan_sub(double* S, double* aux, int n_act = kSub
 #pragma unroll
   for (int o = 0; o < kOwn; ++o)
     if (warp + o * kWarps < panels) gj_store_strip<Ld>(g[o], S, kGJPanel * (warp + o * kWarps));
-  // inverse element (j, perm[c]) sits at exchange slot (perm[j], c)
   if (t < n_act) iperm[perm[t]] = t;
-  __syncthreads();
+  order.perm = perm;
+  order.iperm = iperm;
+  return __syncthreads_or(singular);
+}
+template <int Ld, int kThreads>
+__device__ inline bool gauss_jordan_sub(double* S, double* aux, int n_act = kSub) {
+  GJOrder order;
+  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, order, n_act);
   constexpr int kPer = kSub * kSub / kThreads;
   double x[kPer];
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
-    const int e = t + u * kThreads, j = e / kSub, m = e % kSub;
-    x[u] = (j < n_act && m < n_act) ? S[perm[j] * Ld + iperm[m]] : (j == m ? 1.0 : 0.0);
+    const int e = threadIdx.x + u * kThreads, j = e / kSub, m = e % kSub;
+    x[u] = (j < n_act && m < n_act) ? S[order.perm[j] * Ld + order.iperm[m]] : (j == m ? 1.0 : 0.0);
   }
-  singular = __syncthreads_or(singular);
+  __syncthreads();
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
-    const int e = t + u * kThreads;
+    const int e = threadIdx.x + u * kThreads;
     S[(e / kSub) * Ld + e % kSub] = x[u];
   }
   __syncthreads();
