@@ -387,6 +387,195 @@ __global__ void __launch_bounds__(256, 2) ldmd_elementwise_kernel(int phase, int
   }
 }
 
+// ---- matrices of at most 128 rows: the whole call in one launch ----------------------------------------
+// A sweep of so small a matrix is one CTA's work, and launched pass by pass it is mostly launches, fills of idle SMs and
+// traffic of padding (a 24-row matrix was padded to 128 rows in memory): 27 us per half-step of 21 channels.  Here
+// one CTA keeps its (block, energy) matrix in shared memory through every sector of the call: the elementwise passes
+// run between inversions on the tile itself, and only W, Q_mid, y1 and y2 are read.  D = 32 or 64: Gauss-Jordan
+// exchange, whose permuted result the next pass reads in place; D = 128: the two-level sweep_block.
+// Measured (B200), propagate_logD of N = 21, 1 energy, 16 sectors: 898 -> 397 us a call; coupled-states blocks of 1 to 21
+// channels, 16 energies, 12 sectors: 5.7 -> 4.1 ms a call (the rest is the host's per-block work).
+template <int D>
+struct SmallShape {
+  static constexpr int kThreads = D == 32 ? 128 : 256;
+  static constexpr int kLd = D + 4;
+  static constexpr size_t kAux = D == 128 ? kPivotAuxBytes / sizeof(double) : kGJAuxDoubles;
+  static constexpr size_t kSmemBytes = (size_t(D) * kLd + kAux + 6 * D) * sizeof(double);
+  static constexpr int kPer = D == 128 ? 1 : D * D / kThreads;
+  static constexpr int kPerSM = D == 32 ? 4 : D == 64 ? 2 : 1;
+};
+
+// Invert the matrix in S (used rows: `used`); get(r, c) of the functor passed on is then the swept value
+// -A^{-1}(r, c), symmetrised.  put(r, c, f) for every (r, c) < n_act replaces the matrix by f(r, c, swept value).
+template <int D, class F>
+__device__ inline bool small_sweep_then(double* S, double* aux, int used, F&& f) {
+  using Sh = SmallShape<D>;
+  const int n_act = (int)round_up(used, kGJPanel);
+  if constexpr (D == 128) {
+    const bool singular = sweep_block<true>(S, aux, n_act);
+    // pairs (r, c), (c, r) belong to one thread: in place
+    for (int e = threadIdx.x; e < used * D; e += Sh::kThreads) {
+      const int r = e / D, c = e % D;
+      if (c > r) continue;
+      const double v = 0.5 * (S[r * Sh::kLd + c] + S[c * Sh::kLd + r]);
+      f(r, c, v);
+    }
+    __syncthreads();
+    return singular;
+  } else {
+    GJOrder order;
+    const bool singular = gauss_jordan_exchange<Sh::kLd, Sh::kThreads, D>(S, aux, order, n_act);
+    double x[Sh::kPer];
+#pragma unroll
+    for (int u = 0; u < Sh::kPer; ++u) {
+      const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;
+      x[u] = 0.0;
+      if (r < used && c <= r) x[u] = -0.5 * (S[order.perm[r] * Sh::kLd + order.iperm[c]] + S[order.perm[c] * Sh::kLd + order.iperm[r]]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < Sh::kPer; ++u) {
+      const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;
+      if (r < used && c <= r) f(r, c, x[u]);
+    }
+    __syncthreads();
+    return singular;
+  }
+}
+
+// Both elements of a pair; the identity (once: sweeping leaves +-1 there, decoupled) on the rows from `used` to the edge.
+template <int D>
+__device__ __forceinline__ void small_put(double* S, int r, int c, double v) {
+  S[r * SmallShape<D>::kLd + c] = v;
+  S[c * SmallShape<D>::kLd + r] = v;
+}
+template <int D>
+__device__ __forceinline__ void small_pad(double* S, int used) {
+  const int n_act = D == 128 ? D : (int)round_up(used, kGJPanel);
+  for (int e = threadIdx.x; e < n_act * n_act; e += SmallShape<D>::kThreads) {
+    const int r = e / n_act, c = e % n_act;
+    if (r >= used || c >= used) S[r * SmallShape<D>::kLd + c] = (r == c) ? 1.0 : 0.0;
+  }
+}
+
+// Q_mid of every (sector, block): one CTA each.
+template <int D>
+__global__ void __launch_bounds__(SmallShape<D>::kThreads, SmallShape<D>::kPerSM) ldmd_small_qmid_kernel(LdmdSectors sec, int n, int n_block, int npr, double* Qm, int* status) {
+  extern __shared__ __align__(16) double smem[];
+  using Sh = SmallShape<D>;
+  double* S = smem;
+  double* aux = smem + D * Sh::kLd;
+  const int sg = blockIdx.x, s = sg / n_block, g = sg % n_block;
+  const double h = sec.h[s];
+  const double* Wm = sec.Wm + s * sec.wm_stride + g * sec.wb_stride;
+  double* Q = Qm + (long long)sg * npr * npr;
+  small_pad<D>(S, n);
+  for (int e = threadIdx.x; e < n * n; e += Sh::kThreads) {
+    const int i = e / n, j = e % n;
+    S[i * Sh::kLd + j] = (i == j) ? 1.0 : -h * h * sym(Wm, n, i, j) / 6.0;
+  }
+  __syncthreads();
+  const bool singular = small_sweep_then<D>(S, aux, n, [&](int i, int j, double v) {
+    const double q = 4.0 / h * (-v - (i == j ? 1.0 : 0.0));
+    Q[(long long)i * npr + j] = q;
+    Q[(long long)j * npr + i] = q;
+  });
+  if (singular && threadIdx.x == 0) report_status(status, kDeviceSingularPivot, sg, 0);
+}
+
+template <int D>
+__global__ void __launch_bounds__(SmallShape<D>::kThreads, SmallShape<D>::kPerSM) ldmd_small_kernel(LdmdSectors sec, LdmdLayout L, double* Y, int* status) {
+  extern __shared__ __align__(16) double smem[];
+  using Sh = SmallShape<D>;
+  double* S = smem;
+  double* aux = smem + D * Sh::kLd;
+  double* vec = aux + Sh::kAux;  // ref, y1, y2 of this sector and the one before
+  const int b = blockIdx.x, g = b / L.n_energy, n = L.n, batch = L.n_block * L.n_energy;
+  const bool cplx = L.is_complex != 0;
+  const int used = cplx ? 2 * n : n;
+  bool singular = false;
+  small_pad<D>(S, used);
+  double* Yb = Y + (long long)b * n * n * (cplx ? 2 : 1);
+  for (int s = 0; s < sec.n_sector; ++s) {
+    double *ref = vec + 3 * D * (s & 1), *y1 = ref + D, *y2 = y1 + D;
+    const double *refp = vec + 3 * D * ((s + 1) & 1), *y1p = refp + D, *y2p = y1p + D;
+    const double h = sec.h[s], hp = s > 0 ? sec.h[s - 1] : 0.0;
+    const long long wb = g * sec.wb_stride;
+    const double *Ws = sec.Ws + s * sec.ws_stride + wb, *Wm = sec.Wm + s * sec.wm_stride + wb;
+    const double *We = sec.We + s * sec.we_stride + wb, *Wep = s > 0 ? sec.We + (s - 1) * sec.we_stride + wb : We;
+    const double* Q = L.Qm + ((long long)s * L.n_block + g) * L.npr * L.npr;
+    for (int i = threadIdx.x; i < n; i += Sh::kThreads) {
+      ref[i] = Wm[(long long)i * n + i];
+      y1[i] = L.y1[((long long)s * batch + b) * n + i];
+      y2[i] = L.y2[((long long)s * batch + b) * n + i];
+    }
+    __syncthreads();
+    // element (r, c) of the work matrix: the real part of logical (i, j), or in a complex call the part that its
+    // place in the 2x2 block [[X, Z], [Z, -X]] asks for
+    const auto start = [&](int r, int c, double before) {  // phases 0 and 1: `before` is Y, or y2 S y2 of the last sector
+      const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+      const bool imag = cplx && ((r ^ c) & 1);
+      const double d = (i == j) ? 1.0 : 0.0;
+      double x = before;
+      if (!imag) {
+        if (s > 0) x += hp * (Wep[(long long)i * n + j] - d * refp[i]) / 3.0 + d * y1p[i];
+        x += h * (Ws[(long long)i * n + j] - d * ref[i]) / 3.0 + d * y1[i];
+      }
+      small_put<D>(S, r, c, (cplx && !imag && (r & 1)) ? -x : x);
+    };
+    // y2_i S_ij y2_j from the swept element of the same place (in a complex call -S on the imaginary places and on the
+    // lower right one of each block)
+    const auto folded = [&](int r, int c, double v, const double* w) {
+      if (!cplx) return w[r] * v * w[c];
+      const bool imag = (r ^ c) & 1, lower = !imag && (r & 1);
+      return w[r >> 1] * (imag || lower ? -v : v) * w[c >> 1];
+    };
+    if (s == 0) {
+      for (int e = threadIdx.x; e < used * used; e += Sh::kThreads) {
+        const int r = e / used, c = e % used;
+        if (c > r) continue;
+        double v;
+        if (cplx) {
+          const int i = r >> 1, j = c >> 1, im = (r ^ c) & 1;
+          v = 0.5 * (Yb[2 * ((long long)i * n + j) + im] + Yb[2 * ((long long)j * n + i) + im]);
+        } else {
+          v = 0.5 * (Yb[(long long)r * n + c] + Yb[(long long)c * n + r]);
+        }
+        start(r, c, v);
+      }
+      __syncthreads();
+    } else {
+      singular |= small_sweep_then<D>(S, aux, used, [&](int r, int c, double v) { start(r, c, folded(r, c, v, y2p)); });
+    }
+    singular |= small_sweep_then<D>(S, aux, used, [&](int r, int c, double v) {
+      const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+      const bool imag = cplx && ((r ^ c) & 1);
+      double x = folded(r, c, v, y2);
+      if (!imag) x += 2.0 * Q[(long long)i * L.npr + j] + (i == j ? 2.0 * y1[i] : 0.0);
+      small_put<D>(S, r, c, (cplx && !imag && (r & 1)) ? -x : x);
+    });
+    if (s + 1 == sec.n_sector) {
+      singular |= small_sweep_then<D>(S, aux, used, [&](int r, int c, double v) {
+        const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+        const bool imag = cplx && ((r ^ c) & 1);
+        if (cplx && (r & 1) && !(imag && i == j)) return;  // the first row of each 2x2 block holds both parts (on the diagonal its
+                                                           // imaginary part is visited in the second)
+        const double d = (i == j) ? 1.0 : 0.0;
+        double x = folded(r, c, v, y2);
+        if (!imag) x += h * (We[(long long)i * n + j] - d * ref[i]) / 3.0 + d * y1[i];
+        if (cplx) {
+          Yb[2 * ((long long)i * n + j) + (imag ? 1 : 0)] = x;
+          Yb[2 * ((long long)j * n + i) + (imag ? 1 : 0)] = x;
+        } else {
+          Yb[(long long)i * n + j] = x;
+          Yb[(long long)j * n + i] = x;
+        }
+      });
+    }
+  }
+  if (singular && threadIdx.x == 0) report_status(status, kDeviceSingularPivot, b, 0);
+}
+
 inline unsigned grid_for(long long work, int threads, unsigned cap = 1u << 16) {
   long long blocks = (work + threads - 1) / threads;
   if (blocks < 1) blocks = 1;
@@ -411,6 +600,23 @@ inline cudaError_t ldmd_qmid(const LdmdSectors& sec, LdmdLayout& L, int* status,
   return cudaGetLastError();
 }
 
+template <int D>
+inline cudaError_t ldmd_small_qmid(const LdmdSectors& sec, const LdmdLayout& L, int* status, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(ldmd_small_qmid_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SmallShape<D>::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  ldmd_small_qmid_kernel<D><<<sec.n_sector * L.n_block, SmallShape<D>::kThreads, SmallShape<D>::kSmemBytes, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm, status);
+  note_launch();
+  return cudaGetLastError();
+}
+template <int D>
+inline cudaError_t ldmd_small(double* Y, const LdmdSectors& sec, const LdmdLayout& L, int* status, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(ldmd_small_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SmallShape<D>::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  ldmd_small_kernel<D><<<L.n_block * L.n_energy, SmallShape<D>::kThreads, SmallShape<D>::kSmemBytes, stream>>>(sec, L, Y, status);
+  note_launch();
+  return cudaGetLastError();
+}
+
 // Propagate every (block, energy) through every sector of the call.  Y (device,
 // n_block x n_energy x n x n, complex interleaved when is_complex) is read at the first
 // sector start and overwritten with the log-derivative at the last sector end.
@@ -421,6 +627,12 @@ inline cudaError_t ldmd_propagate(double* Y, const double* energies, double mu, 
   if (L.reduced != nullptr) {
     ldmd_reduced_blocks_kernel<<<sec.n_sector, 256, 0, stream>>>(sec, energies, mu, L.n, L.n_energy, L.n_block, L.np, L.is_complex, L.reduced);
     note_launch();
+  }
+  const int rows = L.is_complex ? 2 * L.n : L.n;
+  if (rows <= kBlock) {
+    cudaError_t e = L.n <= 32 ? ldmd_small_qmid<32>(sec, L, status, stream) : L.n <= 64 ? ldmd_small_qmid<64>(sec, L, status, stream) : ldmd_small_qmid<128>(sec, L, status, stream);
+    if (e != cudaSuccess) return e;
+    return rows <= 32 ? ldmd_small<32>(Y, sec, L, status, stream) : rows <= 64 ? ldmd_small<64>(Y, sec, L, status, stream) : ldmd_small<128>(Y, sec, L, status, stream);
   }
   cudaError_t err = ldmd_qmid(sec, L, status, stream);
   if (err != cudaSuccess) return err;

@@ -39,35 +39,36 @@ constexpr size_t kPivotSmemBytes = size_t(kBlock) * kPivotLd * sizeof(double) + 
 constexpr size_t kUpdateSmemBytes = kUpdTileSmemBytes + 16;  // + the broadcast slot of the tile queue  // stages + C tile; the pivot aux reuses the stages
 static_assert(kPivotAuxBytes <= size_t(kUpdStageDoubles) * sizeof(double), "pivot scratch must fit in the update stages");
 
-// One warp's 8-column strip of a 64x64 block in DMMA accumulator layout: lane l holds row 8 mt + l / 4, columns
+// One warp's 8-column strip of a D x D block (D = 32 or 64) in DMMA accumulator layout: lane l holds row 8 mt + l / 4, columns
 // 2 (l % 4) and the next, for every 8-row tile mt.
+template <int D>
 struct GJStrip {
-  double2 v[kSub / 8];
+  double2 v[D / 8];
 };
-template <int Ld>
-__device__ __forceinline__ void gj_load_strip(GJStrip& g, const double* S, int c0) {
+template <int Ld, int D>
+__device__ __forceinline__ void gj_load_strip(GJStrip<D>& g, const double* S, int c0) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int mt = 0; mt < kSub / 8; ++mt) g.v[mt] = *reinterpret_cast<const double2*>(S + (8 * mt + (lane >> 2)) * Ld + c0 + 2 * (lane & 3));
+  for (int mt = 0; mt < D / 8; ++mt) g.v[mt] = *reinterpret_cast<const double2*>(S + (8 * mt + (lane >> 2)) * Ld + c0 + 2 * (lane & 3));
 }
-template <int Ld>
-__device__ __forceinline__ void gj_store_strip(const GJStrip& g, double* S, int c0) {
+template <int Ld, int D>
+__device__ __forceinline__ void gj_store_strip(const GJStrip<D>& g, double* S, int c0) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int mt = 0; mt < kSub / 8; ++mt) *reinterpret_cast<double2*>(S + (8 * mt + (lane >> 2)) * Ld + c0 + 2 * (lane & 3)) = g.v[mt];
+  for (int mt = 0; mt < D / 8; ++mt) *reinterpret_cast<double2*>(S + (8 * mt + (lane >> 2)) * Ld + c0 + 2 * (lane & 3)) = g.v[mt];
 }
 
 // Panel update of a strip (columns c0 ..): new = (pivot row ? 0 : old) - E W with E the finished panel (columns j0 ..
 // j0 + 7 of S, all rows) and W the strip's old pivot rows, which pass through the strip's place in S.  No branch per row
 // (a divergent one costs some 50 cycles), and no full store of the strip (eight of them at once took the shared-memory
 // pipe 500 cycles): predicated stores.
-template <int Ld>
-__device__ __forceinline__ void gj_update_strip(GJStrip& g, double* S, const int* prow, int c0, int j0, unsigned long long rows_used) {
+template <int Ld, int D>
+__device__ __forceinline__ void gj_update_strip(GJStrip<D>& g, double* S, const int* prow, int c0, int j0, unsigned long long rows_used) {
   const int lane = threadIdx.x & 31, mr = lane >> 2, kr = lane & 3;
   const unsigned lo = (unsigned)rows_used >> mr, hi = (unsigned)(rows_used >> 32) >> mr;
   const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(S + mr * Ld + c0 + 2 * kr));
 #pragma unroll
-  for (int mt = 0; mt < kSub / 8; ++mt) {
+  for (int mt = 0; mt < D / 8; ++mt) {
     const unsigned is_pivot = ((mt < 4 ? lo : hi) >> (8 * (mt & 3))) & 1u;
     asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.v2.f64 [%1], {%2, %3}; }" ::"r"(is_pivot), "r"(at + (unsigned)(8 * mt * Ld * sizeof(double))), "d"(g.v[mt].x), "d"(g.v[mt].y)
                  : "memory");
@@ -78,7 +79,7 @@ __device__ __forceinline__ void gj_update_strip(GJStrip& g, double* S, const int
   const double w0 = -S[prow[kr] * Ld + c0 + mr], w1 = -S[prow[4 + kr] * Ld + c0 + mr];
   const double* e = S + mr * Ld + j0 + kr;
 #pragma unroll
-  for (int mt = 0; mt < kSub / 8; ++mt) {
+  for (int mt = 0; mt < D / 8; ++mt) {
     double acc[2] = {g.v[mt].x, g.v[mt].y};
     dmma_8x8x4(acc, e[8 * mt * Ld], w0);
     dmma_8x8x4(acc, e[8 * mt * Ld + 4], w1);
@@ -97,19 +98,19 @@ __device__ __forceinline__ double gj_reciprocal(double a) {
 }
 
 // Eliminate the panel of columns j0 .. j0 + 7 of S by one warp (exchange steps inside the panel only).  Lane l holds
-// rows l and l + 32; rows in `rows_before` have been pivots (or do not take part).  Returns the panel's pivot rows as
+// rows l and, where D = 64, l + 32; rows in `rows_before` have been pivots (or do not take part).  Returns the panel's pivot rows as
 // a mask; prow[0..7] gets them in order.
-template <int Ld>
+template <int Ld, int D>
 __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* prow, int j0, unsigned long long rows_before, bool& singular) {
   const int lane = threadIdx.x & 31;
   // rank of a row: its magnitude's leading 24 bits, then its index (the smaller row wins); 0 for a used row
   constexpr unsigned kRankMask = ~127u;
-  unsigned mask0 = ((rows_before >> lane) & 1ull) ? 0u : kRankMask, mask1 = ((rows_before >> (lane + 32)) & 1ull) ? 0u : kRankMask;
+  unsigned mask0 = ((rows_before >> lane) & 1ull) ? 0u : kRankMask, mask1 = D == 32 || ((rows_before >> (lane + 32)) & 1ull) ? 0u : kRankMask;
   unsigned code0 = mask0 ? 127u - lane : 0u, code1 = mask1 ? 95u - lane : 0u;
   double v0[kGJPanel], v1[kGJPanel];
 #pragma unroll
   for (int i = 0; i < kGJPanel; i += 2) {
-    const double2 x = *reinterpret_cast<const double2*>(S + lane * Ld + j0 + i), y = *reinterpret_cast<const double2*>(S + (lane + 32) * Ld + j0 + i);
+    const double2 x = *reinterpret_cast<const double2*>(S + lane * Ld + j0 + i), y = *reinterpret_cast<const double2*>(S + (lane + D - 32) * Ld + j0 + i);
     v0[i] = x.x;
     v0[i + 1] = x.y;
     v1[i] = y.x;
@@ -120,7 +121,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
 #pragma unroll 1
   for (int jj = 0; jj < kGJPanel; ++jj) {
     const unsigned h0 = (((unsigned)__double2hiint(v0[0]) << 1) & mask0) | code0, h1 = (((unsigned)__double2hiint(v1[0]) << 1) & mask1) | code1;
-    const bool second = h1 > h0;
+    const bool second = D == 64 && h1 > h0;
     const unsigned key = second ? h1 : h0;
     const unsigned best = __reduce_max_sync(0xffffffffu, key);
     constexpr unsigned kFirst = 1u << 21, kSpan = 0xffe00000u - kFirst;  // ranks of normal finite magnitudes
@@ -129,7 +130,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
     for (int i = 0; i < kGJPanel; ++i) c[i] = second ? v1[i] : v0[i];
     const double inv_own = gj_reciprocal((key - kFirst) < kSpan ? c[0] : 1.0);  // of every lane's candidate, beside the search
     const int row = 127 - (int)(best & 127u);
-    const bool own0 = row == lane, own1 = row == lane + 32;
+    const bool own0 = row == lane, own1 = D == 64 && row == lane + 32;
     mask0 = own0 ? 0u : mask0;
     code0 = own0 ? 0u : code0;
     mask1 = own1 ? 0u : mask1;
@@ -138,10 +139,10 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
 #pragma unroll
     for (int i = 1; i < kGJPanel; ++i) {
       v0[i] = own0 ? 0.0 : v0[i];
-      v1[i] = own1 ? 0.0 : v1[i];
+      if (D == 64) v1[i] = own1 ? 0.0 : v1[i];
     }
     v0[0] = own0 ? 1.0 : v0[0];
-    v1[0] = own1 ? 1.0 : v1[0];
+    if (D == 64) v1[0] = own1 ? 1.0 : v1[0];
     singular |= !((best - kFirst) < kSpan);
     if (lane == 0) prow[jj] = row;
     const double inv = __shfl_sync(0xffffffffu, inv_own, row & 31);
@@ -152,7 +153,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
 #pragma unroll
     for (int i = 0; i + 1 < kGJPanel; ++i) {
       v0[i] = fma(-f0, p[i + 1], v0[i + 1]);
-      v1[i] = fma(-f1, p[i + 1], v1[i + 1]);
+      if (D == 64) v1[i] = fma(-f1, p[i + 1], v1[i + 1]);
     }
     v0[kGJPanel - 1] = f0;
     v1[kGJPanel - 1] = f1;
@@ -160,13 +161,14 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
 #pragma unroll
   for (int i = 0; i < kGJPanel; i += 2) {
     *reinterpret_cast<double2*>(S + lane * Ld + j0 + i) = make_double2(v0[i], v0[i + 1]);
-    *reinterpret_cast<double2*>(S + (lane + 32) * Ld + j0 + i) = make_double2(v1[i], v1[i + 1]);
+    if (D == 64) *reinterpret_cast<double2*>(S + (lane + 32) * Ld + j0 + i) = make_double2(v1[i], v1[i + 1]);
   }
-  const unsigned long long all = ((unsigned long long)__ballot_sync(0xffffffffu, mask1 == 0u) << 32) | __ballot_sync(0xffffffffu, mask0 == 0u);
+  unsigned long long all = __ballot_sync(0xffffffffu, mask0 == 0u);
+  if (D == 64) all |= (unsigned long long)__ballot_sync(0xffffffffu, mask1 == 0u) << 32;
   return all & ~rows_before;
 }
 
-// S <- S^{-1} (64x64 in shared memory, row stride Ld = 4 mod 16) by Gauss-Jordan exchange with partial pivoting over
+// S <- S^{-1} (D x D in shared memory, D = 32 or 64, row stride Ld = 4 mod 16) by Gauss-Jordan exchange with partial pivoting over
 // the block's rows, by the kThreads threads of the CTA.  `n_act` (a multiple of kGJPanel): rows and columns at or beyond
 // it hold the identity and are left alone.  Returns true if a pivot was zero or non-finite.  Uses named barrier 1.
 //
@@ -184,19 +186,19 @@ struct GJOrder {
   const int* perm;
   const int* iperm;
 };
-template <int Ld, int kThreads>
-__device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& order, int n_act = kSub) {
-  constexpr int kWarps = kThreads / 32, kOwn = kSub / kGJPanel / kWarps;
+template <int Ld, int kThreads, int D = kSub>
+__device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& order, int n_act = D) {
+  constexpr int kWarps = kThreads / 32, kOwn = D / kGJPanel / kWarps;
   unsigned long long* panel_rows = reinterpret_cast<unsigned long long*>(aux);  // [kSub / kGJPanel]
   int* perm = reinterpret_cast<int*>(aux + kSub / kGJPanel);
   int* iperm = perm + kSub;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   bool singular = false;
   const int panels = n_act / kGJPanel;
-  unsigned long long used = n_act == kSub ? 0ull : ~0ull << n_act;  // rows of all panels so far
-  GJStrip g[kOwn];
+  unsigned long long used = n_act == 64 ? 0ull : ~0ull << n_act;  // rows of all panels so far
+  GJStrip<D> g[kOwn];
 #pragma unroll
-  for (int o = 0; o < kOwn; ++o) gj_load_strip<Ld>(g[o], S, kGJPanel * (warp + o * kWarps));
+  for (int o = 0; o < kOwn; ++o) gj_load_strip<Ld, D>(g[o], S, kGJPanel * (warp + o * kWarps));
   __syncwarp();
 #pragma unroll 1
   for (int q = -1; q < panels; ++q) {
@@ -213,13 +215,13 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
 #pragma unroll
         for (int o = 0; o < kOwn; ++o)
           if (next == warp + o * kWarps) {
-            gj_update_strip<Ld>(g[o], S, perm + j0, kGJPanel * next, j0, mask);
-            gj_store_strip<Ld>(g[o], S, kGJPanel * next);
+            gj_update_strip<Ld, D>(g[o], S, perm + j0, kGJPanel * next, j0, mask);
+            gj_store_strip<Ld, D>(g[o], S, kGJPanel * next);
           }
         asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
         __syncwarp();
       }
-      const unsigned long long m = gj_factor_panel<Ld>(S, perm + j0 + kGJPanel, j0 + kGJPanel, used, singular);
+      const unsigned long long m = gj_factor_panel<Ld, D>(S, perm + j0 + kGJPanel, j0 + kGJPanel, used, singular);
       if (lane == 0) panel_rows[q + 1] = m;
     } else if (more && q >= 0) {
       asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");  // the next panel's owner has the tensor pipe to itself
@@ -228,14 +230,14 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
 #pragma unroll
     for (int o = 0; o < kOwn; ++o) {
       const int strip = warp + o * kWarps;
-      if (strip == q) gj_load_strip<Ld>(g[o], S, j0);
-      else if (strip < panels && !(mine && strip == next)) gj_update_strip<Ld>(g[o], S, perm + j0, kGJPanel * strip, j0, mask);
+      if (strip == q) gj_load_strip<Ld, D>(g[o], S, j0);
+      else if (strip < panels && !(mine && strip == next)) gj_update_strip<Ld, D>(g[o], S, perm + j0, kGJPanel * strip, j0, mask);
     }
   }
   __syncthreads();  // the last panel's E has been read
 #pragma unroll
   for (int o = 0; o < kOwn; ++o)
-    if (warp + o * kWarps < panels) gj_store_strip<Ld>(g[o], S, kGJPanel * (warp + o * kWarps));
+    if (warp + o * kWarps < panels) gj_store_strip<Ld, D>(g[o], S, kGJPanel * (warp + o * kWarps));
   if (t < n_act) iperm[perm[t]] = t;
   order.perm = perm;
   order.iperm = iperm;
@@ -298,9 +300,9 @@ __device__ inline void small_gemm64(double* C, int ldc, const double* A, int lda
 // Sweep the 128x128 block held in shared memory (row stride kPivotLd) in place:
 // P <- -P^{-1}, through its two 64-wide sub-blocks (the same principal pivot transform
 // as the outer sweep, one level down).  aux holds a 64 x kSmallLd temporary and the
-// Gauss-Jordan bookkeeping.
+// Gauss-Jordan bookkeeping; rows from `n_act` (a multiple of kGJPanel, above 64) on are decoupled and +-1.
 template <bool kSym>
-__device__ inline bool sweep_block(double* P, double* aux) {
+__device__ inline bool sweep_block(double* P, double* aux, int n_act = kBlock) {
   double* U = aux;
   double* gj = aux + kSub * kSmallLd;
   bool singular = false;
@@ -310,7 +312,7 @@ __device__ inline bool sweep_block(double* P, double* aux) {
     double* Pkr = P + k0 * kPivotLd + r0;
     double* Prk = P + r0 * kPivotLd + k0;
     double* Prr = P + r0 * kPivotLd + r0;
-    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj);
+    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj, s == 0 ? kSub : n_act - kSub);
     small_gemm64(U, kSmallLd, Pkk, kPivotLd, Pkr, kPivotLd, 1.0, false);     // U = P_KK^-1 P_KR
     small_gemm64(Prr, kPivotLd, Prk, kPivotLd, U, kSmallLd, -1.0, true);  // P_RR -= P_RK U
     if (!kSym) small_gemm64(Prk, kPivotLd, Prk, kPivotLd, Pkk, kPivotLd, 1.0, false);  // V = P_RK P_KK^-1
