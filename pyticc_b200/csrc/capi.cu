@@ -400,43 +400,50 @@ int ticc_pes_legendre_grid(const double* R, int n_R, const double* r, int n_r, c
 }
 
 // ---- BF -> SF transform ------------------------------------------------------------------------------
-static size_t transform_layout(int n, int batch, double** Bp, double** P, double** T, char* base) {
+static size_t transform_layout(int n, int batch, double** Bp, double** P, double** T, int** lists, char* base) {
   Carver c{base};
   const int np = ticc::ldmd_np(n, 0);
   *Bp = c.take<double>((size_t)np * np);
   *P = c.take<double>((size_t)batch * np * np);
   *T = c.take<double>((size_t)batch * np * np);
+  *lists = c.take<int>(4 + (size_t)(np / ticc::kBlock) * (np / ticc::kChunk + 1));  // non-finite flag, chunk lists
   return c.used + 256;
 }
 
 int ticc_transform_workspace_size(int n, int batch, int is_complex, size_t* bytes) {
   if (n < 1 || batch < 1 || bytes == nullptr) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_transform_workspace_size: n=%d batch=%d", n, batch);
   double *a, *b, *c;
-  *bytes = transform_layout(n, batch, &a, &b, &c, nullptr);
+  int* d;
+  *bytes = transform_layout(n, batch, &a, &b, &c, &d, nullptr);
   return TICC_OK;
 }
 
 int ticc_transform_bf_to_sf(const void* Y, void* Y_out, const double* B, int n, int batch, int is_complex, void* workspace, size_t workspace_bytes, void* stream) {
   if (Y == nullptr || Y_out == nullptr || B == nullptr || n < 1 || batch < 1) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_transform_bf_to_sf: bad arguments");
   double *Bp, *P, *T;
-  const size_t need = transform_layout(n, batch, &Bp, &P, &T, nullptr);
+  int* flag;
+  const size_t need = transform_layout(n, batch, &Bp, &P, &T, &flag, nullptr);
   if (workspace == nullptr || workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "ticc_transform_bf_to_sf: workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-  transform_layout(n, batch, &Bp, &P, &T, static_cast<char*>(workspace));
+  transform_layout(n, batch, &Bp, &P, &T, &flag, static_cast<char*>(workspace));
+  int* lists = flag + 4;
   const int np = ticc::ldmd_np(n, 0);
   cudaStream_t s = as_stream(stream);
   const long long area = (long long)np * np;
   ticc::pad_plane_kernel<<<dim3(ticc::grid_for(area, 256, 8192), 1), 256, 0, s>>>(B, n, 0, 0, Bp, np);
   ticc::note_launch();
   for (int part = 0; part < (is_complex ? 2 : 1); ++part) {
-    ticc::pad_plane_kernel<<<dim3(ticc::grid_for(area, 256, 8192), batch), 256, 0, s>>>(static_cast<const double*>(Y), n, is_complex, part, P, np);
+    cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
+    if (e != cudaSuccess) return cuda_fail(e, "ticc_transform_bf_to_sf");
+    ticc::pad_plane_kernel<<<dim3(ticc::grid_for(area, 256, 8192), batch), 256, 0, s>>>(static_cast<const double*>(Y), n, is_complex, part, P, np, flag);
     ticc::note_launch();
-    // T^T = (B^T Y)^T, then (B^T T^T)^T = T B = B^T Y B
-    ticc::GemmBatch g1{Bp, np, 0, P, np, area, T, np, area, np, 1.0, 1};
-    cudaError_t e = ticc::gemm_tn(g1, np, np, batch, s);
-    if (e != cudaSuccess) return cuda_fail(e, "ticc_transform_bf_to_sf");
-    ticc::GemmBatch g2{Bp, np, 0, T, np, area, P, np, area, np, 1.0, 1};
-    e = ticc::gemm_tn(g2, np, np, batch, s);
-    if (e != cudaSuccess) return cuda_fail(e, "ticc_transform_bf_to_sf");
+    // T^T = (B^T Y)^T, then (B^T T^T)^T = T B = B^T Y B, over the row chunks of B that hold non-zeros
+    for (int half = 0; half < 2; ++half) {
+      ticc::chunk_list_kernel<<<np / ticc::kBlock, ticc::kListThreads, 0, s>>>(Bp, np, np, flag, lists);
+      ticc::note_launch();
+      const ticc::GemmBatch g{Bp, np, 0, half == 0 ? P : T, np, area, half == 0 ? T : P, np, area, np, 1.0, 1, lists, flag};
+      e = ticc::gemm_tn(g, np, np, batch, s);
+      if (e != cudaSuccess) return cuda_fail(e, "ticc_transform_bf_to_sf");
+    }
     ticc::unpad_plane_kernel<<<dim3(ticc::grid_for((long long)n * n, 256, 8192), batch), 256, 0, s>>>(P, np, static_cast<double*>(Y_out), n, is_complex, part);
     ticc::note_launch();
   }

@@ -69,8 +69,9 @@ __device__ __forceinline__ void mma_chunk(TileAcc& acc, const double* As, const 
 }
 
 // acc = sum_{k < K} A[k][0..127]^T B[k][0..127]; A, B already offset to their tile column.
-// K must be a multiple of kChunk.  Ends with a __syncthreads(), so smem is free afterwards.
-__device__ inline void tile_gemm_tn(TileAcc& acc, const double* A, long long lda, const double* B, long long ldb, int K, double* smem) {
+// K must be a multiple of kChunk.  With `list`, only the `listed` chunks of kChunk rows that it names (ascending).
+// Ends with a __syncthreads(), so smem is free afterwards.
+__device__ inline void tile_gemm_tn(TileAcc& acc, const double* A, long long lda, const double* B, long long ldb, int K, double* smem, const int* list = nullptr, int listed = 0) {
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
@@ -81,15 +82,20 @@ __device__ inline void tile_gemm_tn(TileAcc& acc, const double* A, long long lda
 
   // stage s of the double buffer: A at smem + s * 2 * kChunk * kStride, B right after it
   constexpr int kStage = 2 * kChunk * kStride;
-  const int nchunks = K / kChunk;
-  stage_rows(smem, A, lda, 0, tid);
-  stage_rows(smem + kChunk * kStride, B, ldb, 0, tid);
-  cp_async_commit();
+  const int nchunks = list != nullptr ? listed : K / kChunk;
+  const auto row_of = [&](int c) { return (list != nullptr ? list[c] : c) * kChunk; };
+  if (nchunks > 0) {
+    const int k = row_of(0);
+    stage_rows(smem, A, lda, k, tid);
+    stage_rows(smem + kChunk * kStride, B, ldb, k, tid);
+    cp_async_commit();
+  }
   for (int c = 0; c < nchunks; ++c) {
     if (c + 1 < nchunks) {
       double* next = smem + ((c + 1) & 1) * kStage;
-      stage_rows(next, A, lda, (c + 1) * kChunk, tid);
-      stage_rows(next + kChunk * kStride, B, ldb, (c + 1) * kChunk, tid);
+      const int k = row_of(c + 1);
+      stage_rows(next, A, lda, k, tid);
+      stage_rows(next + kChunk * kStride, B, ldb, k, tid);
       cp_async_commit();
       cp_async_wait<1>();
     } else {
