@@ -1,8 +1,8 @@
 // Bessel functions of real order for asymptotic matching, in FP64, on the device.
 //
 // J_nu, Y_nu and their derivatives (nu >= 0, x > 0) follow Steed's method:
-//   * CF1: f = J'_nu / J_nu from the continued fraction of the ratios J_{nu+k}/J_{nu+k-1}
-//     (modified Lentz); the product of the signs of its denominators is sign(J_nu);
+//   * CF1: f = J'_nu / J_nu from the continued fraction of the ratios J_{nu+k}/J_{nu+k-1} (Wallis' recurrence of
+//     its convergents, modified Lentz for tiny x); the sign of the last denominator is sign(J_nu);
 //   * downward recurrence from nu to mu = nu - nl (|mu| <= 1/2 for x < 2);
 //   * x >= 2: CF2, the complex continued fraction for (J'_mu + iY'_mu)/(J_mu + iY_mu),
 //     closed with the Wronskian J Y' - J' Y = 2/(pi x);
@@ -91,24 +91,58 @@ TICC_HD inline BesselJY bessel_jy(double nu, double x) {
   if (nl < 0) nl = 0;
   const double mu = nu - nl;
 
-  // CF1
-  double f = (nu / x > tiny) ? nu / x : tiny;
-  double C = f, D = 0.0;
+  // CF1: f = nu/x - 1/(b_1 - 1/(b_2 - ...)), b_k = 2 (nu + k)/x
+  double f;
   int sign = 1;
-  int k = 1;
-  for (; k < kBesselMaxIter; ++k) {
-    const double b = 2.0 * (nu + k) / x;
-    D = b - D;
-    if (fabs(D) < tiny) D = tiny;
-    C = b - 1.0 / C;
-    if (fabs(C) < tiny) C = tiny;
-    D = 1.0 / D;
-    const double delta = C * D;
-    f *= delta;
-    if (D < 0.0) sign = -sign;
-    if (fabs(delta - 1.0) < stop) break;
+  if (x < 1.0e-3) {  // modified Lentz: a few terms, whose size would overflow the plain recurrence
+    f = (nu / x > tiny) ? nu / x : tiny;
+    double C = f, D = 0.0;
+    int k = 1;
+    for (; k < kBesselMaxIter; ++k) {
+      const double b = 2.0 * (nu + k) / x;
+      D = b - D;
+      if (fabs(D) < tiny) D = tiny;
+      C = b - 1.0 / C;
+      if (fabs(C) < tiny) C = tiny;
+      D = 1.0 / D;
+      const double delta = C * D;
+      f *= delta;
+      if (D < 0.0) sign = -sign;
+      if (fabs(delta - 1.0) < stop) break;
+    }
+    if (k >= kBesselMaxIter) return out;
+  } else {
+    // the convergents' numerators and denominators by their linear recurrence (Wallis): no division in the chain, where
+    // Lentz's method takes two dependent ones a term, and about x terms are needed.  A convergent is formed every 16
+    // terms; past k ~ x they converge faster than geometrically, so agreement of two of them leaves rounding only.
+    // 2/x in two parts: a rounded one would be the same relative error in every term, that is, a shifted phase
+    const double step = 2.0 / x, step_lo = fma(-step, x, 2.0) / x;
+    double A0 = 1.0, A1 = nu / x, B0 = 0.0, B1 = 1.0;
+    f = A1;
+    int k = 0;
+    for (; k < kBesselMaxIter; k += 16) {
+      for (int i = 1; i <= 16; ++i) {
+        const double nk = nu + (k + i), b = fma(step, nk, step_lo * nk);
+        const double A2 = b * A1 - A0, B2 = b * B1 - B0;
+        A0 = A1;
+        A1 = A2;
+        B0 = B1;
+        B1 = B2;
+        if (fabs(B1) > 1.0e200 || fabs(A1) > 1.0e200) {
+          A0 *= 1.0e-200;
+          A1 *= 1.0e-200;
+          B0 *= 1.0e-200;
+          B1 *= 1.0e-200;
+        }
+      }
+      const double next = A1 / B1;
+      const bool done = fabs(next - f) <= 16.0 * stop * fabs(next);
+      f = next;
+      if (done) break;
+    }
+    if (k >= kBesselMaxIter) return out;
+    sign = (B1 < 0.0) ? -1 : 1;
   }
-  if (k >= kBesselMaxIter) return out;
 
   // downward recurrence of (J, J') from nu to mu, with rescaling
   double Jl = sign, Jpl = f * Jl, lam = nu;
@@ -267,6 +301,40 @@ TICC_HD inline double bessel_k_ratio(double nu, double x) {
   }
   return sb / sa;
 }
+
+#ifdef __CUDACC__
+// The same ratio by one warp (all lanes call it with the same arguments): 32 terms of the sums a turn, away from the peak in
+// both directions until a whole turn is below exp(-60) of it.
+__device__ inline double bessel_k_ratio_warp(double nu, double x) {
+  const int lane = threadIdx.x & 31;
+  const double a = fabs(nu), b = fabs(nu - 1.0);
+  const double kap = sqrt(hypot(x, a));
+  const double h = fmin(0.1, 0.25 / fmax(1.0, kap));
+  const double tstar = asinh(a / x);
+  const double pmax = -x * (cosh(tstar) - 1.0) + a * tstar;
+  const long long k0 = (long long)(tstar / h);
+  double sa = 0.0, sb = 0.0;
+  for (int dir = 0; dir < 2; ++dir) {
+    for (int it = 0;; ++it) {
+      if (it > kBesselMaxIter / 32) return NAN;
+      const long long k = dir == 0 ? k0 + 32LL * it + lane : k0 - 1 - 32LL * it - lane;
+      bool small = true;
+      if (k >= 0) {
+        const double t = k * h, w = (k == 0) ? 0.5 : 1.0;
+        sa += w * k_integrand(x, t, a, pmax);
+        sb += w * k_integrand(x, t, b, pmax);
+        small = -x * (cosh(t) - 1.0) + a * t < pmax - 60.0;
+      }
+      if (__all_sync(0xffffffffu, small)) break;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    sa += __shfl_xor_sync(0xffffffffu, sa, o);
+    sb += __shfl_xor_sync(0xffffffffu, sb, o);
+  }
+  return sb / sa;
+}
+#endif
 
 // K'_nu(x)/K_nu(x) = -K_{nu-1}(x)/K_nu(x) - nu/x.
 TICC_HD inline double bessel_k_logd(double nu, double x) { return -bessel_k_ratio(nu, x) - nu / x; }

@@ -1437,8 +1437,8 @@ inline cudaError_t sweep_sym(double* M, long long mstride, int np, int batch, do
                              float* split = nullptr) {
   return sweep_batched<true>(M, mstride, np, batch, scratch, status, stream, reduced_blocks, n_used, split);
 }
-inline cudaError_t sweep_general(double* M, long long mstride, int np, int batch, double* scratch, int* status, cudaStream_t stream) {
-  return sweep_batched<false>(M, mstride, np, batch, scratch, status, stream);
+inline cudaError_t sweep_general(double* M, long long mstride, int np, int batch, double* scratch, int* status, cudaStream_t stream, int n_used = 0) {
+  return sweep_batched<false>(M, mstride, np, batch, scratch, status, stream, nullptr, n_used);
 }
 
 }  // namespace ticc
