@@ -186,205 +186,213 @@ __device__ __forceinline__ void get_swept(const double* Mb, int np, int i, int j
 // Work-matrix padding: identity on the padded diagonal of the real sweep matrix.
 __device__ __forceinline__ void put_padding(double* Mb, int np, long long r, long long c) { Mb[r * np + c] = (r == c) ? 1.0 : 0.0; }
 
-// W_base must be exactly symmetric (the contraction writes both halves from one value), so
-// the per-energy passes read W[i][j] only, row-contiguous across the threads of a warp.
+// W_base must be exactly symmetric (the contraction writes both halves from one value), so the per-energy passes read
+// W[i][j] only, row-contiguous across the lanes of a warp.
 // phase 0: A = Y_in + Q_start + y1          (first sector of the call)
 // phase 1: A = [Q_end' + y1' + y2' S y2'] + Q_start + y1   (S from the previous sector)
 // phase 2: B = 2 Q_mid + 2 y1 + y2 S y2
 // phase 3: Y_out = Q_end + y1 + y2 S y2     (last sector of the call)
-// One CTA per (logical row i, channel block g) runs over every energy of the block: the
-// row's W (or Q_mid) values are read once into registers and reused for all energies, and
-// each thread keeps kRowCols columns of loads in flight per energy.  Every quantity is
-// symmetric in (i, j) and the sweep reads only the lower and diagonal 128-tiles, so a row
-// is processed up to the end of its diagonal tile; the last pass writes Y_out's upper
-// triangle as the transpose of the lower tiles.
-constexpr int kRowCols = 4;
-__global__ void __launch_bounds__(256, 2) ldmd_elementwise_kernel(int phase, int s, LdmdSectors sec, LdmdLayout L, const double* Yin, double* Yout) {
-  const int i = blockIdx.x;
-  const int g = blockIdx.y;
-  const int ne = L.n_energy;
-  const int batch = L.n_block * ne;
-  const int n = L.n, np = L.np;
-  const int nl = L.is_complex ? np / 2 : np;  // logical-element grid covering the padded matrix
-  const int mi = L.is_complex ? 2 * i : i;    // work-matrix row of logical row i
-  const int tile_end = ((mi >> 7) + 1) << 7;  // end of row i's diagonal 128-tile (work-matrix columns)
-  const int jl = L.is_complex ? tile_end / 2 : tile_end;
-  const int jlim = jl < nl ? jl : nl;
-  if (i >= n) {  // padding row
-    if (phase == 3) return;
-    for (int e = 0; e < ne; ++e) {
-      double* Mb = L.M + (long long)(g * ne + e) * np * np;
-      for (int j = threadIdx.x; j < jlim; j += blockDim.x) {
-        if (L.is_complex) {
-          for (int a = 0; a < 2; ++a)
-            for (int c = 0; c < 2; ++c) put_padding(Mb, np, 2LL * i + a, 2LL * j + c);
-        } else {
-          put_padding(Mb, np, i, j);
-        }
-      }
-    }
-    return;
-  }
+// Every quantity is symmetric and the sweep reads only the lower and diagonal 128-tiles, so only those are passed over: bound by
+// reading and writing them once.  A CTA covers 16 logical rows of one 128-tile (a warp two rows, a lane two double2
+// of each: two columns of a real matrix, one element X + iZ of a complex one) for a group of energies; the
+// energy-independent part of its elements stays in registers over the group, and two energies' loads are in flight at a
+// time.  The groups are cut so that few or small matrices still fill the chip (one CTA a row over all energies took
+// 15 us for 16 matrices of 231 channels and 350 us for 16 of 1984 in phase 2: here 7 and 97, 5.9 TB/s).  Y_in and Y_out are dense
+// n x n; their transposed halves pass through shared memory in 16-column strips.
+constexpr int kElemRows = 16;
+constexpr int kElemThreads = 256;
+
+template <int kPhase, bool kCplx>
+__global__ void __launch_bounds__(kElemThreads) ldmd_elementwise_kernel(int s, int e_per, LdmdSectors sec, LdmdLayout L, const double* Yin, double* Yout) {
+  constexpr int kCols = kCplx ? kBlock / 2 : kBlock;     // logical columns (and rows) of a 128-tile
+  constexpr int kGroups = kCols / kElemRows;             // row groups of a tile
+  constexpr int kEach = kCplx ? 1 : 2;                   // logical columns of a double2
+  constexpr bool kDense = kPhase == 0 || kPhase == 3;    // reads or writes Y
+  // [logical column of the tile][row of the group]: the transposed half of Y, one plane for each part of a complex element
+  __shared__ double strip[kDense ? (kCplx ? 2 : 1) * kCols * (kElemRows + 1) : 1];
+  int ta, tb;
+  lower_pair(blockIdx.x / kGroups, ta, tb);
+  const int g = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = L.n, np = L.np, ne = L.n_energy, batch = L.n_block * ne;
+  const int i0 = ta * kCols + (blockIdx.x % kGroups) * kElemRows, j0 = tb * kCols;
+  const int e0 = blockIdx.y * e_per, e1 = min(ne, e0 + e_per);
+  if (kPhase == 3 && i0 >= n) return;
   const double h = sec.h[s];
   const long long wb = g * sec.wb_stride;
-  const double* Ws = sec.Ws + s * sec.ws_stride + wb + (long long)i * n;
   const double* Wm = sec.Wm + s * sec.wm_stride + wb;
-  const double* We = sec.We + s * sec.we_stride + wb + (long long)i * n;
-  const double ref = Wm[(long long)i * n + i];
-  double hp = 0.0, ref_p = 0.0;
-  const double* Wep = nullptr;
-  if (phase == 1) {
-    hp = sec.h[s - 1];
-    Wep = sec.We + (s - 1) * sec.we_stride + wb + (long long)i * n;
-    ref_p = sec.Wm[(s - 1) * sec.wm_stride + wb + (long long)i * n + i];
-  }
-  const double* Qrow = L.Qm + ((long long)s * L.n_block + g) * L.npr * L.npr + (long long)i * L.npr;
-  for (int j0 = 0; j0 < jlim; j0 += kRowCols * 256) {
-    // energy-independent row values of this thread's columns
-    double wa[kRowCols], wp[kRowCols];
+  const int i[2] = {i0 + 2 * warp, i0 + 2 * warp + 1};
+  // energy-independent part of each element: [row][chunk][column of the double2]
+  double base[2][2][kEach];
+  const double* Wrow = (kPhase == 3 ? sec.We + s * sec.we_stride : sec.Ws + s * sec.ws_stride) + wb;
+  const double* Wprev = kPhase == 1 ? sec.We + (s - 1) * sec.we_stride + wb : nullptr;
+  const double* Q = L.Qm + ((long long)s * L.n_block + g) * L.npr * L.npr;
+  const double h3 = h / 3.0, hp3 = kPhase == 1 ? sec.h[s - 1] / 3.0 : 0.0;
 #pragma unroll
-    for (int q = 0; q < kRowCols; ++q) {
-      const int j = j0 + q * 256 + threadIdx.x;
-      wa[q] = wp[q] = 0.0;
-      if (j < n) {
-        if (phase <= 1) wa[q] = Ws[j];
-        else if (phase == 2) wa[q] = Qrow[j];
-        else wa[q] = We[j];
-        if (phase == 1) wp[q] = Wep[j];
-      }
+  for (int r = 0; r < 2; ++r) {
+    double ref = 0.0, ref_p = 0.0;  // taken off the diagonal before anything is multiplied: W_ii - ref_i cancels
+    if (kPhase != 2 && i[r] < n) {
+      ref = Wm[(long long)i[r] * n + i[r]];
+      if (kPhase == 1) ref_p = sec.Wm[(s - 1) * sec.wm_stride + wb + (long long)i[r] * n + i[r]];
     }
-    if (!L.is_complex && (phase == 1 || phase == 2)) {
-      // the per-sector passes of a real work matrix: two energies at a time, all loads of
-      // both issued before either's stores (the stores of one energy could alias the next
-      // energy's loads as far as the compiler knows, so it would not hoist them itself)
-#pragma unroll 1
-      for (int e = 0; e < ne; e += 2) {
-        const int cnt = (ne - e < 2) ? ne - e : 2;
-        double sv[2][kRowCols], yv[2][kRowCols], y1i[2], y2i[2];
-        double* Mv[2];
-        const double* y2row[2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int b = g * ne + e + (u < cnt ? u : 0);
-          Mv[u] = L.M + (long long)b * np * np;
-          const double* y1 = L.y1 + ((long long)(phase == 1 ? s - 1 : s) * batch + b) * n;
-          y2row[u] = L.y2 + ((long long)(phase == 1 ? s - 1 : s) * batch + b) * n;
-          y1i[u] = y1[i];
-          y2i[u] = y2row[u][i];
+    for (int q = 0; q < 2; ++q)
 #pragma unroll
-          for (int q = 0; q < kRowCols; ++q) {
-            const int j = j0 + q * 256 + threadIdx.x;
-            sv[u][q] = yv[u][q] = 0.0;
-            if (j < n && j < jlim) {
-              sv[u][q] = Mv[u][(long long)i * np + j];
-              yv[u][q] = y2row[u][j];
-            }
+      for (int c = 0; c < kEach; ++c) {
+        const int j = j0 + (q * 32 + lane) * kEach + c;
+        double v = 0.0;
+        if (i[r] < n && j < n) {
+          if (kPhase == 2) {
+            v = 2.0 * Q[(long long)i[r] * L.npr + j];
+          } else {
+            v = h3 * (Wrow[(long long)i[r] * n + j] - (i[r] == j ? ref : 0.0));
+            if (kPhase == 1) v = fma(hp3, Wprev[(long long)i[r] * n + j] - (i[r] == j ? ref_p : 0.0), v);
           }
         }
+        base[r][q][c] = v;
+      }
+  }
+  const int sy = kPhase == 1 ? s - 1 : s;  // the sector whose y1, y2 fold the swept matrix
+  for (int e = e0; e < e1; e += 2) {
+    const int cnt = min(2, e1 - e);
+    double2 m[2][2][2];  // [energy][row][chunk]: swept values in, new values out
+    double yj[2][2][kEach];
+    if (kPhase != 0) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (u >= cnt) break;
-          const int b = g * ne + e + u;
-          const double* y1c = L.y1 + ((long long)s * batch + b) * n;  // this sector's y1 (phase 1)
-          const double y1cur = y1c[i];
+      for (int u = 0; u < 2; ++u) {
+        const int b = g * ne + e + (u < cnt ? u : 0);
+        const double* Mb = L.M + (long long)b * np * np + (long long)j0 * (kCplx ? 2 : 1);
+        const double* y2 = L.y2 + ((long long)sy * batch + b) * n;
 #pragma unroll
-          for (int q = 0; q < kRowCols; ++q) {
-            const int j = j0 + q * 256 + threadIdx.x;
-            if (j >= jlim) continue;
-            if (j >= n) {  // padding column
-              put_padding(Mv[u], np, i, j);
-              continue;
-            }
-            const double d = (i == j) ? 1.0 : 0.0;
-            double x;
-            if (phase == 1) {
-              x = hp * (wp[q] - d * ref_p) / 3.0 + d * y1i[u] + y2i[u] * sv[u][q] * yv[u][q];
-              x += h * (wa[q] - d * ref) / 3.0 + d * y1cur;
+        for (int q = 0; q < 2; ++q) {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) m[u][r][q] = *reinterpret_cast<const double2*>(Mb + (long long)(kCplx ? 2 * i[r] : i[r]) * np + (q * 32 + lane) * 2);
+#pragma unroll
+          for (int c = 0; c < kEach; ++c) {
+            const int j = j0 + (q * 32 + lane) * kEach + c;
+            yj[u][q][c] = j < n ? y2[j] : 0.0;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u >= cnt) break;
+      const int b = g * ne + e + u;
+      const double* Yb = Yin + (long long)b * n * n * (kCplx ? 2 : 1);
+      if (kPhase == 0) {  // Y[j][i] of the group's rows, 16 contiguous columns a row
+        __syncthreads();
+        for (int t = threadIdx.x; t < kCols * kElemRows; t += kElemThreads) {
+          const int jj = t / kElemRows, ii = t % kElemRows;
+          const bool in = j0 + jj < n && i0 + ii < n;
+          const long long at = (long long)(j0 + jj) * n + i0 + ii;
+          if (kCplx) {
+            strip[jj * (kElemRows + 1) + ii] = in ? Yb[2 * at] : 0.0;
+            strip[(kCols + jj) * (kElemRows + 1) + ii] = in ? Yb[2 * at + 1] : 0.0;
+          } else {
+            strip[jj * (kElemRows + 1) + ii] = in ? Yb[at] : 0.0;
+          }
+        }
+        __syncthreads();
+      }
+      if (kPhase == 3) __syncthreads();  // the previous energy's strip has been written out
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const bool row_in = i[r] < n;
+        const double* y1 = L.y1 + ((long long)s * batch + b) * n;
+        const double y1i = row_in ? y1[i[r]] : 0.0;
+        const double y2i = row_in && kPhase != 0 ? L.y2[((long long)sy * batch + b) * n + i[r]] : 0.0;
+        const double d = kPhase == 2 ? 2.0 * y1i : kPhase == 1 ? y1i + (row_in ? L.y1[((long long)sy * batch + b) * n + i[r]] : 0.0) : y1i;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int j = j0 + (q * 32 + lane) * kEach, jj = j - j0, ii = i[r] - i0;
+          double2 x;
+          if (kCplx) {
+            const bool in = row_in && j < n;
+            x = make_double2(base[r][q][0] + (i[r] == j ? d : 0.0), 0.0);
+            if (kPhase == 0) {
+              const long long at = (long long)i[r] * n + j;
+              if (in) {
+                x.x += 0.5 * (Yb[2 * at] + strip[jj * (kElemRows + 1) + ii]);
+                x.y = 0.5 * (Yb[2 * at + 1] + strip[(kCols + jj) * (kElemRows + 1) + ii]);
+              }
             } else {
-              x = 2.0 * wa[q] + 2.0 * d * y1i[u] + y2i[u] * sv[u][q] * yv[u][q];
+              x.x += y2i * m[u][r][q].x * yj[u][q][0];
+              x.y = -(y2i * m[u][r][q].y * yj[u][q][0]);  // the embedding holds -S on its imaginary places
             }
-            Mv[u][(long long)i * np + j] = x;
+            if (!in) x = make_double2(i[r] == j ? 1.0 : 0.0, 0.0);
+          } else {
+            x = make_double2(base[r][q][0] + (i[r] == j ? d : 0.0), base[r][q][kEach - 1] + (i[r] == j + 1 ? d : 0.0));
+            if (kPhase == 0) {
+              const long long at = (long long)i[r] * n + j;
+              if (row_in && j < n) x.x += 0.5 * (Yb[at] + strip[jj * (kElemRows + 1) + ii]);
+              if (row_in && j + 1 < n) x.y += 0.5 * (Yb[at + 1] + strip[(jj + 1) * (kElemRows + 1) + ii]);
+            } else {
+              x.x += y2i * m[u][r][q].x * yj[u][q][0];
+              x.y += y2i * m[u][r][q].y * yj[u][q][kEach - 1];
+            }
+            if (!row_in || j >= n) x.x = (i[r] == j) ? 1.0 : 0.0;
+            if (!row_in || j + 1 >= n) x.y = (i[r] == j + 1) ? 1.0 : 0.0;
+          }
+          if (kPhase != 3) {
+            double* Mb = L.M + (long long)b * np * np + (long long)j0 * (kCplx ? 2 : 1) + (q * 32 + lane) * 2;
+            if (kCplx) {
+              const bool pad = !row_in || j >= n;
+              *reinterpret_cast<double2*>(Mb + (long long)(2 * i[r]) * np) = x;
+              *reinterpret_cast<double2*>(Mb + (long long)(2 * i[r] + 1) * np) = pad ? make_double2(0.0, x.x) : make_double2(x.y, -x.x);
+            } else {
+              *reinterpret_cast<double2*>(Mb + (long long)i[r] * np) = x;
+            }
+          } else {
+            double* Yo = Yout + (long long)b * n * n * (kCplx ? 2 : 1);
+            const long long at = (long long)i[r] * n + j;
+            if (kCplx) {
+              if (row_in && j < n) *reinterpret_cast<double2*>(Yo + 2 * at) = x;
+              strip[jj * (kElemRows + 1) + ii] = x.x;
+              strip[(kCols + jj) * (kElemRows + 1) + ii] = x.y;
+            } else {
+              if (row_in && j < n) Yo[at] = x.x;
+              if (row_in && j + 1 < n) Yo[at + 1] = x.y;
+              strip[jj * (kElemRows + 1) + ii] = x.x;
+              strip[(jj + 1) * (kElemRows + 1) + ii] = x.y;
+            }
           }
         }
       }
-      continue;
-    }
-#pragma unroll 1
-    for (int e = 0; e < ne; ++e) {
-      const int b = g * ne + e;
-      double* Mb = L.M + (long long)b * np * np;
-      const double* y1 = L.y1 + ((long long)s * batch + b) * n;
-      const double* y2 = L.y2 + ((long long)s * batch + b) * n;
-      const double y1i = y1[i], y2i = y2[i];
-      double y1pi = 0.0, y2pi = 0.0;
-      const double* y2p = nullptr;
-      if (phase == 1) {
-        const double* y1p = L.y1 + ((long long)(s - 1) * batch + b) * n;
-        y2p = L.y2 + ((long long)(s - 1) * batch + b) * n;
-        y1pi = y1p[i];
-        y2pi = y2p[i];
-      }
-#pragma unroll
-      for (int q = 0; q < kRowCols; ++q) {
-        const int j = j0 + q * 256 + threadIdx.x;
-        if (j >= jlim) continue;
-        if (j >= n) {  // padding column
-          if (phase == 3) continue;
-          if (L.is_complex) {
-            for (int a = 0; a < 2; ++a)
-              for (int c = 0; c < 2; ++c) put_padding(Mb, np, 2LL * i + a, 2LL * j + c);
-          } else {
-            put_padding(Mb, np, i, j);
-          }
-          continue;
-        }
-        const double d = (i == j) ? 1.0 : 0.0;
-        double x = 0.0, z = 0.0;
-        if (phase == 0) {
-          if (L.is_complex) {
-            const double* Yb = Yin + (long long)b * n * n * 2;
-            x = 0.5 * (Yb[2 * ((long long)i * n + j)] + Yb[2 * ((long long)j * n + i)]);
-            z = 0.5 * (Yb[2 * ((long long)i * n + j) + 1] + Yb[2 * ((long long)j * n + i) + 1]);
-          } else {
-            const double* Yb = Yin + (long long)b * n * n;
-            x = 0.5 * (Yb[(long long)i * n + j] + Yb[(long long)j * n + i]);
-          }
-        } else if (phase == 1) {
-          double sr, si;
-          get_swept(Mb, np, i, j, L.is_complex, sr, si);
-          x = hp * (wp[q] - d * ref_p) / 3.0 + d * y1pi + y2pi * sr * y2p[j];
-          z = y2pi * si * y2p[j];
-        }
-        if (phase <= 1) {
-          x += h * (wa[q] - d * ref) / 3.0 + d * y1i;
-          put_element(Mb, np, i, j, x, z, L.is_complex);
-        } else if (phase == 2) {
-          double sr, si;
-          get_swept(Mb, np, i, j, L.is_complex, sr, si);
-          x = 2.0 * wa[q] + 2.0 * d * y1i + y2i * sr * y2[j];
-          z = y2i * si * y2[j];
-          put_element(Mb, np, i, j, x, z, L.is_complex);
-        } else {
-          double sr, si;
-          get_swept(Mb, np, i, j, L.is_complex, sr, si);
-          x = h * (wa[q] - d * ref) / 3.0 + d * y1i + y2i * sr * y2[j];
-          z = y2i * si * y2[j];
-          const bool below = ((L.is_complex ? 2 * j : j) >> 7) < (mi >> 7);  // (i, j) in a strictly lower tile
-          if (L.is_complex) {
-            Yout[((long long)b * n * n + (long long)i * n + j) * 2] = x;
-            Yout[((long long)b * n * n + (long long)i * n + j) * 2 + 1] = z;
-            if (below) {
-              Yout[((long long)b * n * n + (long long)j * n + i) * 2] = x;
-              Yout[((long long)b * n * n + (long long)j * n + i) * 2 + 1] = z;
-            }
-          } else {
-            Yout[(long long)b * n * n + (long long)i * n + j] = x;
-            if (below) Yout[(long long)b * n * n + (long long)j * n + i] = x;
-          }
+      if (kPhase == 3 && ta != tb) {  // the upper half as the transpose of the lower tiles
+        __syncthreads();
+        double* Yo = Yout + (long long)b * n * n * (kCplx ? 2 : 1);
+        for (int t = threadIdx.x; t < kCols * kElemRows; t += kElemThreads) {
+          const int jj = t / kElemRows, ii = t % kElemRows;
+          if (j0 + jj >= n || i0 + ii >= n) continue;
+          const long long at = (long long)(j0 + jj) * n + i0 + ii;
+          if (kCplx) *reinterpret_cast<double2*>(Yo + 2 * at) = make_double2(strip[jj * (kElemRows + 1) + ii], strip[(kCols + jj) * (kElemRows + 1) + ii]);
+          else Yo[at] = strip[jj * (kElemRows + 1) + ii];
         }
       }
     }
   }
+}
+
+inline cudaError_t ldmd_elementwise(int phase, int s, const LdmdSectors& sec, const LdmdLayout& L, const double* Yin, double* Yout, cudaStream_t stream) {
+  const int nt = L.np / kBlock, groups = (L.is_complex ? kBlock / 2 : kBlock) / kElemRows;
+  const long long tiles = (long long)nt * (nt + 1) / 2 * groups;
+  // energies of a CTA: all of them where that still gives some six CTAs an SM
+  const long long per_energy = tiles * L.n_block, target = 900;
+  long long e_per = per_energy * L.n_energy / target;
+  e_per = e_per < 1 ? 1 : e_per > L.n_energy ? L.n_energy : e_per;
+  const dim3 grid((unsigned)tiles, (unsigned)((L.n_energy + e_per - 1) / e_per), (unsigned)L.n_block);
+#define TICC_ELEMENTWISE(P)                                                                                                                  \
+  if (L.is_complex) ldmd_elementwise_kernel<P, true><<<grid, kElemThreads, 0, stream>>>(s, (int)e_per, sec, L, Yin, Yout);  \
+  else ldmd_elementwise_kernel<P, false><<<grid, kElemThreads, 0, stream>>>(s, (int)e_per, sec, L, Yin, Yout);
+  switch (phase) {
+    case 0: TICC_ELEMENTWISE(0) break;
+    case 1: TICC_ELEMENTWISE(1) break;
+    case 2: TICC_ELEMENTWISE(2) break;
+    default: TICC_ELEMENTWISE(3) break;
+  }
+#undef TICC_ELEMENTWISE
+  note_launch();
+  return cudaGetLastError();
 }
 
 // ---- matrices of at most 128 rows: the whole call in one launch ----------------------------------------
@@ -636,24 +644,20 @@ inline cudaError_t ldmd_propagate(double* Y, const double* energies, double mu, 
   }
   cudaError_t err = ldmd_qmid(sec, L, status, stream);
   if (err != cudaSuccess) return err;
-  const long long nl = L.is_complex ? L.np / 2 : L.np;
-  const dim3 grid((unsigned)nl, L.n_block);
   const long long mstride = (long long)L.np * L.np;
   const int used = L.is_complex ? 2 * L.n : L.n;  // rows of the work matrix beyond these are identity padding
   FineState fine{L.fine};
   for (int s = 0; s < sec.n_sector; ++s) {
-    ldmd_elementwise_kernel<<<grid, 256, 0, stream>>>(s == 0 ? 0 : 1, s, sec, L, Y, Y);
-    note_launch();
+    err = ldmd_elementwise(s == 0 ? 0 : 1, s, sec, L, Y, Y, stream);
+    if (err != cudaSuccess) return err;
     err = sweep_any(fine, L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
     if (err != cudaSuccess) return err;
-    ldmd_elementwise_kernel<<<grid, 256, 0, stream>>>(2, s, sec, L, Y, Y);
-    note_launch();
+    err = ldmd_elementwise(2, s, sec, L, Y, Y, stream);
+    if (err != cudaSuccess) return err;
     err = sweep_any(fine, L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
     if (err != cudaSuccess) return err;
   }
-  ldmd_elementwise_kernel<<<grid, 256, 0, stream>>>(3, sec.n_sector - 1, sec, L, Y, Y);
-  note_launch();
-  return cudaGetLastError();
+  return ldmd_elementwise(3, sec.n_sector - 1, sec, L, Y, Y, stream);
 }
 
 }  // namespace ticc
