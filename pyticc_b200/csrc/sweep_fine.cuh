@@ -16,8 +16,8 @@
 // Flags (per matrix, monotonic over the sweeps of one call, so that only the first one clears them): per lower tile the number
 // of steps applied, per block row the last panel, the last inverted pivot, per step the finished updates (a
 // panel slot is rewritten kFineSlots steps later, once its readers are done).
-// A step of the chain takes 26-28 us: 15 for the block's inversion, 2.3 for each of its two products (one SM's FP64 pipe),
-// 3 for publishing P^{-1}, 1.4 for the flag and the next CTA's loads.
+// A step of the chain takes 24-25 us: 15 for the block's inversion, 2.3 for each of its two products (one SM's FP64 pipe),
+// 2 for publishing P^{-1}, the rest the flag's way to the next CTA, its load of P^{-1} and the stores in between.
 #pragma once
 
 #include <algorithm>
@@ -63,30 +63,31 @@ __device__ __forceinline__ int fine_row_at(int k, int nt, int pos) {
 }
 __device__ __forceinline__ int fine_lower(int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; }
 
-// Thread 0 polls until every flag reaches its target; all threads return whether that happened before the poll
-// limit and without an abort by another CTA.  Ends with a __syncthreads().
+// Thread 0 polls until every flag reaches its target (all flags' loads in flight together: one after the other they cost the
+// chain 2000 cycles a step); all threads return whether that happened before the poll limit and without an abort by
+// another CTA.  Ends with a __syncthreads().
 struct FineNeed {
   const int* flag[4];
   int target[4];
-  int count = 0;
-  __device__ __forceinline__ void add(const int* f, int t) {
-    flag[count] = f;
-    target[count++] = t;
-  }
 };
+__device__ __forceinline__ FineNeed fine_need(const int* f0, int t0, const int* f1, int t1, const int* f2, int t2, const int* f3, int t3) { return FineNeed{{f0, f1, f2, f3}, {t0, t1, t2, t3}}; }
 __device__ inline bool fine_wait(const FineSweep& w, const FineNeed& need, int b, int* shared_ok) {
   if (threadIdx.x == 0) {
     int ok = 1;
     const long long limit = g_step_poll_limit;
     for (long long it = 0;; ++it) {
-      if (it >= limit || load_relaxed(w.control + 1) != 0) {
+      if (it >= limit) {
         if (atomicExch(w.control + 1, 1) == 0) report_status(w.status, kDeviceStalled, b, -1);
         ok = 0;
         break;
       }
-      bool all = true;
-      for (int i = 0; i < need.count; ++i) all = all && load_relaxed(need.flag[i]) >= need.target[i];
-      if (all) {
+      const int abort = load_relaxed(w.control + 1);
+      const int f0 = load_relaxed(need.flag[0]), f1 = load_relaxed(need.flag[1]), f2 = load_relaxed(need.flag[2]), f3 = load_relaxed(need.flag[3]);
+      if (abort != 0) {
+        ok = 0;
+        break;
+      }
+      if (f0 >= need.target[0] && f1 >= need.target[1] && f2 >= need.target[2] && f3 >= need.target[3]) {
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
         break;
       }
@@ -264,17 +265,36 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       const int j = fine_row_at(k, nt, pos);
       const bool below = j > k;  // the lower tile is (j, k), X[c][k]; else (k, j), X[k][c]
       double* T = Mb + (long long)(below ? j : k) * kSub * w.ld + (below ? k : j) * kSub;
-      FineNeed need;
-      need.add(f + 2 * nt, now + 1);
-      need.add(ver + fine_lower(j, k), now);
-      if (k >= kFineSlots) need.add(done + k - kFineSlots, (w.sweep + 1) * per_update);
-      if (chain) need.add(ver + fine_lower(j, j), now);
-      if (!fine_wait(w, need, b, slot + 1)) return;
-      const double* P = w.pinv + ((long long)b * kFinePinv + k % kFinePinv) * kFineTile;
-      for (int half = 0; half < 2; ++half) {
-        fine_stage(SA, T, w.ld, half);
-        fine_stage(SB, P, kSub, half);
+      const int* mine = ver + fine_lower(j, k);
+      const int* pivot = f + 2 * nt;
+      const int* diagonal = chain ? ver + fine_lower(j, j) : mine;
+      const int* readers = k >= kFineSlots ? done + k - kFineSlots : mine;  // the slot's readers kFineSlots steps ago
+      const int readers_target = k >= kFineSlots ? (w.sweep + 1) * per_update : now;
+      double* Xj = X + (long long)j * kFineTile;
+      double* Rj = R + (long long)j * kFineTile;
+      // everything but P^{-1} first: the chain's next link is then only P^{-1} away
+      if (!fine_wait(w, fine_need(mine, now, diagonal, now, readers, readers_target, mine, now), b, slot + 1)) return;
+      for (int half = 0; half < 2; ++half) fine_stage(SA, T, w.ld, half);
+      cp_async_commit();
+      FineAcc old;
+      if (chain) {
+        const double* C = Mb + (long long)j * kSub * w.ld + j * kSub;
+        fine_each(old, [&](int r, int c, double(&d)[2]) {
+          const double2 x = __ldcg(reinterpret_cast<const double2*>(C + (long long)r * w.ld + c));
+          d[0] = x.x;
+          d[1] = x.y;
+        });
       }
+      cp_async_wait<0>();
+      __syncthreads();
+#pragma unroll 4
+      for (int e = tid; e < kFineTile / 2; e += kFineThreads) {
+        const int r = e / (kSub / 2), c = 2 * (e % (kSub / 2));
+        *reinterpret_cast<double2*>(Xj + r * kSub + c) = *reinterpret_cast<const double2*>(SA + r * kSmallLd + c);
+      }
+      if (!fine_wait(w, fine_need(pivot, now + 1, pivot, now + 1, pivot, now + 1, pivot, now + 1), b, slot + 1)) return;
+      const double* P = w.pinv + ((long long)b * kFinePinv + k % kFinePinv) * kFineTile;
+      for (int half = 0; half < 2; ++half) fine_stage(SB, P, kSub, half);
       cp_async_commit();
       cp_async_wait<0>();
       __syncthreads();
@@ -283,13 +303,6 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       // P is symmetric: X P for a tile below the diagonal block (rows of X are its channels), P X for one before it
       if (below) fine_product(acc, SA, kSmallLd, 1, SB, kSmallLd, 1, 0, kSub);
       else fine_product(acc, SB, kSmallLd, 1, SA, kSmallLd, 1, 0, kSub);
-      double* Xj = X + (long long)j * kFineTile;
-      double* Rj = R + (long long)j * kFineTile;
-#pragma unroll 4
-      for (int e = tid; e < kFineTile / 2; e += kFineThreads) {
-        const int r = e / (kSub / 2), c = 2 * (e % (kSub / 2));
-        *reinterpret_cast<double2*>(Xj + r * kSub + c) = *reinterpret_cast<const double2*>(SA + r * kSmallLd + c);
-      }
       const bool mirror = fine_mirrors(below ? j : k, below ? k : j, last);
       double* Mt = Mb + (long long)(below ? k : j) * kSub * w.ld + (below ? j : k) * kSub;
       fine_each(acc, [&](int r, int c, double(&d)[2]) {
@@ -310,13 +323,6 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       }
       if (!chain) continue;
       // M(j, j) - X R^T (here j = k + 1 > k: X[c][k], R[c][k]), lower half, mirrored
-      const double* C = Mb + (long long)j * kSub * w.ld + j * kSub;
-      FineAcc old;
-      fine_each(old, [&](int r, int c, double(&d)[2]) {
-        const double2 x = __ldcg(reinterpret_cast<const double2*>(C + (long long)r * w.ld + c));
-        d[0] = x.x;
-        d[1] = x.y;
-      });
       fine_zero(acc);
       fine_product(acc, SA, kSmallLd, 1, SC, 1, kSmallLd, 0, kSub);
       __syncthreads();
@@ -333,11 +339,8 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
     // ---- trailing update of one lower tile
     const int jx = fine_row_at(k, nt, px), jy = fine_row_at(k, nt, py);
     const int ta = max(jx, jy), tb = min(jx, jy);
-    FineNeed need;
-    need.add(f + ta, now + 1);
-    need.add(f + tb, now + 1);
-    need.add(ver + fine_lower(ta, tb), now);
-    if (!fine_wait(w, need, b, slot + 1)) return;
+    const int* mine = ver + fine_lower(ta, tb);
+    if (!fine_wait(w, fine_need(f + ta, now + 1, f + tb, now + 1, mine, now, mine, now), b, slot + 1)) return;
     const double* Xa = X + (long long)ta * kFineTile;
     const double* Rb = R + (long long)tb * kFineTile;
     for (int half = 0; half < 2; ++half) {
