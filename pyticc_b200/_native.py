@@ -136,7 +136,9 @@ def as_device(value, device: torch.device, dtype: torch.dtype) -> torch.Tensor:
     """Contiguous device tensor of the requested dtype (copies only when needed)."""
     if isinstance(value, torch.Tensor):
         return value.to(device=device, dtype=dtype).contiguous()
-    array = np.array(value, copy=True, order="C")
+    array = np.asarray(value, order="C")
+    if device.type != "cuda" or not array.flags.writeable or not array.flags.c_contiguous:
+        array = np.array(array, copy=True, order="C")  # a CUDA device gets a copy anyway; torch wants writable memory
     if np.iscomplexobj(array) and dtype == torch.float64:
         array = array.real
     return torch.as_tensor(array, device=device, dtype=dtype).contiguous()

@@ -9,6 +9,7 @@ of ``propagation/runner.py:265-271``).
 
 from __future__ import annotations
 
+import ctypes
 from collections.abc import Sequence
 from dataclasses import dataclass, field
 from math import prod
@@ -20,6 +21,9 @@ from numpy.typing import NDArray
 
 from .. import _native as nat
 from ..basis import clebsch_gordan, norm_YjK
+
+
+_INT_P = ctypes.POINTER(ctypes.c_int)
 
 
 @dataclass(frozen=True)
@@ -160,7 +164,9 @@ def contract_rows(rows: DeviceRows, potential: torch.Tensor, *, radial_points: t
     if out is None:
         out = torch.empty((n_R, n, n), dtype=torch.float64, device=dev)
     offsets = rows.group_offsets
-    c_offsets = (nat._I * offsets.size)(*offsets.tolist())
+    if not (offsets.dtype == np.int32 and offsets.flags.c_contiguous):
+        offsets = np.ascontiguousarray(offsets, dtype=np.int32)
+    c_offsets = offsets.ctypes.data_as(_INT_P)
     with torch.cuda.device(dev):
         nat.check(
             lib.ticc_contract(

@@ -117,8 +117,8 @@ def finish_stats(stats: dict) -> dict:
 
 
 def initial_logD(W0: torch.Tensor, energies: torch.Tensor, reduced_mass: float, mode: str) -> torch.Tensor:
-    """Y(R0) from diag W(R0; E) = diag W_base(R0) - 2 mu E (logd.py:48-91)."""
-    d = torch.diagonal(W0)[None, :] - 2.0 * reduced_mass * energies[:, None]
+    """Y(R0) from diag W(R0; E) = diag W_base(R0) - 2 mu E (logd.py:48-91), for one W_base or a batch of them."""
+    d = torch.diagonal(W0, dim1=-2, dim2=-1)[..., None, :] - 2.0 * reduced_mass * energies[:, None]
     if mode == "inelastic":
         return torch.diag_embed(torch.sqrt(torch.abs(d))).contiguous()
     values = torch.where(d >= 0.0, torch.sqrt(torch.clamp(d, min=0.0)).to(torch.complex128), -1j * torch.sqrt(torch.clamp(-d, min=0.0)).to(torch.complex128))
@@ -260,25 +260,22 @@ class DeviceBlocks:
             self.E_int.append(st.E_int)
             self.position.append(st.position)
 
-    def _contract(self, rows, radial_points, U, E_int, out=None):
-        dev = U.device
+    def points(self, radial_points: np.ndarray) -> tuple[torch.Tensor, torch.Tensor]:
+        """The PES rows and radii of a window on the device, shared by every block."""
+        dev = self.values.device
         index = torch.as_tensor(self.grid.selection(radial_points), device=dev)
-        potential = self.values.index_select(0, index)
-        R = torch.as_tensor(np.ascontiguousarray(radial_points), device=dev)
-        return contract_rows(rows, potential, radial_points=R, U=U, E_int=E_int, reduced_mass=self.reduced_mass, out=out)
+        return self.values.index_select(0, index), torch.as_tensor(np.ascontiguousarray(radial_points), device=dev)
 
     def thresholds(self, energies: np.ndarray, device: torch.device) -> list[torch.Tensor]:
-        """Per block E_int padded with the closed padding thresholds for these energies."""
-        dummy = float(np.max(energies)) + DUMMY_P2 / (2.0 * self.reduced_mass)
-        out = []
-        for E_int in self.E_int:
-            padded = np.full(self.n, dummy)
-            padded[: E_int.size] = E_int
-            out.append(torch.as_tensor(padded, device=device))
-        return out
+        """Per block E_int padded with the closed padding thresholds for these energies (rows of one device copy)."""
+        padded = np.full((len(self.E_int), self.n), float(np.max(energies)) + DUMMY_P2 / (2.0 * self.reduced_mass))
+        for row, E_int in zip(padded, self.E_int, strict=True):
+            row[: E_int.size] = E_int
+        return list(torch.as_tensor(padded, device=device).unbind(0))
 
-    def W_base(self, g: int, radial_points: np.ndarray, E_int: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-        return self._contract(self.rows[g], radial_points, self.U[g], E_int, out=out)
+    def W_base(self, g: int, points: tuple[torch.Tensor, torch.Tensor], E_int: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+        potential, R = points
+        return contract_rows(self.rows[g], potential, radial_points=R, U=self.U[g], E_int=E_int, reduced_mass=self.reduced_mass, out=out)
 
 
 def device_blocks(hamiltonian, blocks, device: torch.device, closed_first: bool = False) -> DeviceBlocks:
@@ -365,10 +362,11 @@ def propagate_blocks(hamiltonian, channel_blocks, Etot, radial_sectors: Sequence
     for s0 in range(0, n_sector, size):
         window = tuple(radial_sectors[s0 : s0 + size])
         points = radial_points_of(window)
+        shared = db.points(points)
         for g in range(n_block):
-            db.W_base(g, points, E_pad[g], W[g, : points.size])
+            db.W_base(g, shared, E_pad[g], W[g, : points.size])
         if Y is None:
-            Y = torch.stack([initial_logD(W[g, 0], energies, db.reduced_mass, config.mode) for g in range(n_block)]).contiguous()
+            Y = initial_logD(W[:, 0], energies, db.reduced_mass, config.mode)
         halves = torch.as_tensor(np.asarray([s.radial_half_step for s in window]), device=dev)
         stride = 2 * n * n
         if window_timing is not None:
@@ -385,8 +383,7 @@ def propagate_blocks(hamiltonian, channel_blocks, Etot, radial_sectors: Sequence
             while next_report <= done:
                 next_report += interval
     out = []
-    for g, size_g in enumerate(db.sizes):
-        pos = db.position[g]
-        out.append(Y[g, :, :size_g, :size_g][:, pos][:, :, pos].contiguous())
+    for g, pos in enumerate(db.position):  # propagated index of each block channel: the padding drops out
+        out.append(Y[g][:, pos[:, None], pos])
     return tuple(out)
 
