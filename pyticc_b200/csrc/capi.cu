@@ -305,8 +305,8 @@ int ticc_contract(const double* rows_real, const double* rows_imag, const int* g
   auto flush = [&]() {
     const int n_tiles = tiles.tile_start[tiles.n_groups];
     for (int r0 = 0; r0 < n_R; r0 += 65535) {
-      ticc::contract_group_kernel<<<dim3(n_tiles, std::min(65535, n_R - r0)), 256, ticc::kVSmemBytes, s>>>(tiles, rows_real, rows_imag, row_out, n_grid, scale, potential,
-                                                                                                     pot_stride, r0, n_channel, out);
+      ticc::contract_group_kernel<<<dim3(n_tiles, std::min(65535, n_R - r0)), ticc::kVThreads, ticc::kVSmemBytes, s>>>(tiles, rows_real, rows_imag, row_out, n_grid, scale, potential,
+                                                                                                                 pot_stride, r0, n_channel, out);
       ticc::note_launch();
     }
     tiles.n_groups = 0;
@@ -340,7 +340,7 @@ int ticc_contract_block(const double* A, int n_a, const double* B, int n_b, int 
   if (e != cudaSuccess) return cuda_fail(e, "ticc_contract_block");
   for (int r0 = 0; r0 < n_R; r0 += 65535) {
     const dim3 grid((n_a + ticc::kVTile - 1) / ticc::kVTile, (n_b + ticc::kVTile - 1) / ticc::kVTile, std::min(65535, n_R - r0));
-    ticc::weighted_block_kernel<<<grid, 256, ticc::kVSmemBytes, as_stream(stream)>>>(A, n_a, B, n_b, n_grid, weights, w_stride, r0, pos_a, pos_b, symmetric, mirror, n, out);
+    ticc::weighted_block_kernel<<<grid, ticc::kVThreads, ticc::kVSmemBytes, as_stream(stream)>>>(A, n_a, B, n_b, n_grid, weights, w_stride, r0, pos_a, pos_b, symmetric, mirror, n, out);
     ticc::note_launch();
   }
   e = cudaGetLastError();

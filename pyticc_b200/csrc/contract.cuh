@@ -2,7 +2,7 @@
 //
 // For one K group with weighted rows B (n_K x n_grid) and PES values v(R) on the
 // quadrature grid, V_K(R)[a][b] = norm sum_q (Br[a][q] Br[b][q] + Bi[a][q] Bi[b][q]) v[q].
-// One launch covers every group: each CTA computes a 64x64 lower-triangular tile of one group
+// One launch covers every group: each CTA computes a 32x32 lower-triangular tile of one group
 // at one R on the FP64 tensor pipe and writes both (a, b) and (b, a), so V is exactly symmetric
 // (the reference symmetrises explicitly).  The init kernel writes U/R^2 + 2 mu diag(E_int) (or
 // zeros when only V is wanted) and the group kernel adds 2 mu V (or V) at the rows' output
@@ -31,40 +31,51 @@ __global__ void contract_init_kernel(double* out, int n, int n_R, const double* 
 }
 
 // ---- the weighted-product tile on the FP64 tensor pipe ------------------------------------------
-// A CTA of 8 warps computes one 64 x 64 tile X[i][j] = sum_q A[i][q] w[q] B[j][q] (plus the same
-// over a second pair A2, B2: the imaginary rows of a complex basis) with mma.sync m8n8k4 f64
-// (DMMA), FP64 accumulation.  The rows are read as stored (row-major, q contiguous, any n_grid
-// and any row offset) in chunks of 32 grid points: each warp loads whole 256-byte row segments,
-// the weight is applied to A on the way into shared memory, and rows past the operand's end read
-// as zeros.  Shared tiles are [row][q] with a row stride of 36 doubles, so the fragment loads of a
-// half-warp (rows mr = 0..3, k = 0..3) hit 16 distinct bank pairs.  Chunk c + 1 is fetched into
-// registers while chunk c is multiplied from the other shared buffer (one barrier per chunk).
-// Warp w owns rows (w / 4) * 32 .. +31 and columns (w % 4) * 16 .. +15 of the tile: 4 x 2 DMMA
-// accumulators, element [mt][nt][h] at row (w/4)*32 + 8 mt + lane/4, column (w%4)*16 + 8 nt +
-// 2 (lane%4) + h.
-constexpr int kVTile = 64;
+// A CTA computes one kVTile x kVTile tile X[i][j] = sum_q A[i][q] w[q] B[j][q] (plus the same over a second pair A2, B2: the
+// imaginary rows of a complex basis) with mma.sync m8n8k4 f64 (DMMA), FP64 accumulation.  The rows are read as stored
+// (row-major, q contiguous, any n_grid and any row offset) in chunks of 32 grid points: each warp loads whole 256-byte row
+// segments, the weight is applied to A on the way into shared memory, and rows past the operand's end read as zeros.
+// Shared tiles are [row][q] with a row stride of 36 doubles, so the fragment loads of a half-warp (rows mr = 0..3, k =
+// 0..3) hit 16 distinct bank pairs.  Chunk c + 1 is fetched into registers while chunk c is multiplied from the other
+// shared buffer (one barrier per chunk).
+// kVTile = 32, 4 warps of 16 x 16 (2 x 2 DMMA accumulators), six CTAs an SM.  K groups have 4 to a few hundred rows: a 64-tile
+// (8 warps, three CTAs an SM) multiplies up to half of its work for nothing on ragged groups and the upper halves of diagonal
+// tiles, and leaves small jobs with too few CTAs, while the operand bytes it saves come from L2 either way.  Measured, us,
+// 64 / 32: AB+CD pair, 5 groups of 140-224 rows x 2700 complex points, 33 radii 2281 / 1758; 3 radii 394 / 284; 7 groups of
+// 285-480 rows 4722 / 4732; vibrating A+BC, 31 groups of 4-124 rows x 1024 points, 33 radii 903 / 677; 9 groups of 20-52
+// rows, 21 radii 114 / 76.
+constexpr int kVTile = 32;
+constexpr int kVThreads = 128;
 constexpr int kVChunk = 32;
 constexpr int kVLd = kVChunk + 4;
 constexpr int kVMaxGroups = 128;
-constexpr size_t kVSmemBytes = size_t(2) * 2 * kVTile * kVLd * sizeof(double);  // 73728
 
+constexpr int kVPart = 16;  // rows and columns of a warp's part of the tile
+constexpr int kVLoad = kVTile / (kVThreads / 32);  // rows of a chunk that a warp loads
+constexpr size_t kVSmemBytes = size_t(2) * 2 * kVTile * kVLd * sizeof(double);  // 36864
+
+// Element [mt][nt][h] of a warp's accumulator: row vtile_row() + 8 mt + lane / 4, column vtile_col() + 8 nt + 2 (lane % 4) + h.
 struct VTileAcc {
-  double v[4][2][2];
+  double v[2][2][2];
 };
+__device__ __forceinline__ int vtile_row() { return (threadIdx.x >> 6) * kVPart; }
+__device__ __forceinline__ int vtile_col() { return ((threadIdx.x >> 5) & 1) * kVPart; }
 
-// A, B (and A2, B2) point at the tile's first row; rows at or beyond na (nb) read as zero.
+// A, B (and A2, B2) point at the tile's first row; rows at or beyond na (nb) read as zero.  A warp whose part of the tile
+// is not `wanted` loads with the others but does not multiply.
 __device__ inline void vtile_product(VTileAcc& acc, const double* __restrict__ A, int na, const double* __restrict__ B, int nb, const double* __restrict__ A2,
-                                     const double* __restrict__ B2, int n_grid, const double* __restrict__ w, double* smem) {
+                                     const double* __restrict__ B2, int n_grid, const double* __restrict__ w, double* smem, bool wanted = true) {
+  constexpr int kWarps = kVThreads / 32;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qq = lane, rbase = warp;  // loader: grid point q0 + lane of rows warp + 8 i
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16, kr = lane & 3, mr = lane >> 2;
+  const int qq = lane, rbase = warp;  // loader: grid point q0 + lane of rows warp + kWarps i
+  const int wm = vtile_row(), wn = vtile_col(), kr = lane & 3, mr = lane >> 2;
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) acc.v[mt][nt][0] = acc.v[mt][nt][1] = 0.0;
   const int nq = (n_grid + kVChunk - 1) / kVChunk;
   const int nc = A2 != nullptr ? 2 * nq : nq;
-  double ra[8], rb[8];
+  double ra[kVLoad], rb[kVLoad];
   auto fetch = [&](int c) {
     const bool second = c >= nq;
     const double* sa = second ? A2 : A;
@@ -73,17 +84,17 @@ __device__ inline void vtile_product(VTileAcc& acc, const double* __restrict__ A
     const bool in = q < n_grid;
     const double wq = in ? w[q] : 0.0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = rbase + 8 * i;
+    for (int i = 0; i < kVLoad; ++i) {
+      const int row = rbase + kWarps * i;
       ra[i] = (in && row < na) ? sa[(long long)row * n_grid + q] * wq : 0.0;
       rb[i] = (in && row < nb) ? sb[(long long)row * n_grid + q] : 0.0;
     }
   };
   auto put = [&](double* buf) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      buf[(rbase + 8 * i) * kVLd + qq] = ra[i];
-      buf[kVTile * kVLd + (rbase + 8 * i) * kVLd + qq] = rb[i];
+    for (int i = 0; i < kVLoad; ++i) {
+      buf[(rbase + kWarps * i) * kVLd + qq] = ra[i];
+      buf[kVTile * kVLd + (rbase + kWarps * i) * kVLd + qq] = rb[i];
     }
   };
   fetch(0);
@@ -93,24 +104,26 @@ __device__ inline void vtile_product(VTileAcc& acc, const double* __restrict__ A
     if (c + 1 < nc) fetch(c + 1);
     const double* As = smem + (c & 1) * 2 * kVTile * kVLd;
     const double* Bs = As + kVTile * kVLd;
+    if (wanted) {
 #pragma unroll
-    for (int kk = 0; kk < kVChunk; kk += 4) {
-      double a[4], b[2];
+      for (int kk = 0; kk < kVChunk; kk += 4) {
+        double a[2], b[2];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) a[mt] = As[(wm + mt * 8 + mr) * kVLd + kk + kr];
+        for (int mt = 0; mt < 2; ++mt) a[mt] = As[(wm + mt * 8 + mr) * kVLd + kk + kr];
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) b[nt] = Bs[(wn + nt * 8 + mr) * kVLd + kk + kr];
+        for (int nt = 0; nt < 2; ++nt) b[nt] = Bs[(wn + nt * 8 + mr) * kVLd + kk + kr];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+        for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) dmma_8x8x4(acc.v[mt][nt], a[mt], b[nt]);
+          for (int nt = 0; nt < 2; ++nt) dmma_8x8x4(acc.v[mt][nt], a[mt], b[nt]);
+      }
     }
     if (c + 1 < nc) put(smem + ((c + 1) & 1) * 2 * kVTile * kVLd);
     __syncthreads();
   }
 }
 
-// Lower 64-tiles of every K group in one launch: tile t belongs to the group g with
+// Lower kVTile-tiles of every K group in one launch: tile t belongs to the group g with
 // tile_start[g] <= t < tile_start[g + 1] (only groups with rows are listed).
 struct ContractTiles {
   int n_groups;
@@ -119,10 +132,11 @@ struct ContractTiles {
   int rows[kVMaxGroups];
 };
 
-// grid: (the table's tiles, radial points r_first ..); 256 threads; kVSmemBytes dynamic shared memory.
-__global__ void __launch_bounds__(256) contract_group_kernel(const __grid_constant__ ContractTiles tiles, const double* __restrict__ Br, const double* __restrict__ Bi,
-                                                             const int* __restrict__ row_out, int n_grid, double scale, const double* __restrict__ potential,
-                                                             long long pot_stride, int r_first, int n, double* __restrict__ out) {
+// grid: (the table's tiles, radial points r_first ..).
+__global__ void __launch_bounds__(kVThreads, 6) contract_group_kernel(const __grid_constant__ ContractTiles tiles, const double* __restrict__ Br,
+                                                                                               const double* __restrict__ Bi, const int* __restrict__ row_out, int n_grid, double scale,
+                                                                                               const double* __restrict__ potential, long long pot_stride, int r_first, int n,
+                                                                                               double* __restrict__ out) {
   extern __shared__ __align__(16) double vsmem[];
   const int t = blockIdx.x;
   int g = 0, hi = tiles.n_groups - 1;
@@ -139,14 +153,15 @@ __global__ void __launch_bounds__(256) contract_group_kernel(const __grid_consta
   const int row0 = tiles.row0[g], rows = tiles.rows[g];
   const int r = r_first + blockIdx.y;
   const long long ia = (long long)(row0 + ta * kVTile) * n_grid, ib = (long long)(row0 + tb * kVTile) * n_grid;
+  const int wm = vtile_row(), wn = vtile_col(), lane = threadIdx.x & 31;
+  // a warp's part below the last row, or strictly above the diagonal, adds nothing
+  const bool wanted = ta * kVTile + wm < rows && tb * kVTile + wn < rows && (ta != tb || wm + kVPart > wn);
   VTileAcc acc;
   vtile_product(acc, Br + ia, rows - ta * kVTile, Br + ib, rows - tb * kVTile, Bi != nullptr ? Bi + ia : nullptr, Bi != nullptr ? Bi + ib : nullptr, n_grid,
-                potential + (long long)r * pot_stride, vsmem);
+                   potential + (long long)r * pot_stride, vsmem, wanted);
   double* o = out + (long long)r * n * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -165,9 +180,9 @@ __global__ void __launch_bounds__(256) contract_group_kernel(const __grid_consta
 //     X(R)[i][j] = sum_q A[i][q] w(R)[q] B[j][q],   A: n_a x n_grid, B: n_b x n_grid (row strides n_grid)
 // written to out(R)[pos_a[i]][pos_b[j]] and, with `mirror`, also to out(R)[pos_b[j]][pos_a[i]].
 // A symmetric block (`symmetric`: B is A and pos_b is pos_a) computes only i >= j and writes
-// both (i, j) and (j, i), so the block is exactly symmetric.  grid: (64-tiles of A, 64-tiles of B,
-// radial points r_first ..); 256 threads; kVSmemBytes dynamic shared memory.
-__global__ void __launch_bounds__(256) weighted_block_kernel(const double* __restrict__ A, int n_a, const double* __restrict__ B, int n_b, int n_grid, const double* __restrict__ w,
+// both (i, j) and (j, i), so the block is exactly symmetric.  grid: (tiles of A, tiles of B,
+// radial points r_first ..); kVThreads threads; kVSmemBytes dynamic shared memory.
+__global__ void __launch_bounds__(kVThreads) weighted_block_kernel(const double* __restrict__ A, int n_a, const double* __restrict__ B, int n_b, int n_grid, const double* __restrict__ w,
                                                              long long w_stride, int r_first, const int* __restrict__ pos_a, const int* __restrict__ pos_b, int symmetric,
                                                              int mirror, int n, double* __restrict__ out) {
   extern __shared__ __align__(16) double vsmem[];
@@ -177,10 +192,9 @@ __global__ void __launch_bounds__(256) weighted_block_kernel(const double* __res
   VTileAcc acc;
   vtile_product(acc, A + (long long)i0 * n_grid, n_a - i0, B + (long long)j0 * n_grid, n_b - j0, nullptr, nullptr, n_grid, w + (long long)R * w_stride, vsmem);
   double* o = out + (long long)R * n * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+  const int lane = threadIdx.x & 31, wm = vtile_row(), wn = vtile_col();
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
