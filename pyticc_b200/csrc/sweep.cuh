@@ -33,7 +33,9 @@ constexpr int kPivotLd = kStride;  // the pivot block lives in a [128][kStride] 
 constexpr int kSub = 64;           // Gauss-Jordan sub-block of the pivot block
 constexpr int kSmallLd = kSub + 4; // row stride of a 64-wide shared block: 4 mod 16, conflict-free DMMA fragments
 constexpr int kGJPanel = 8;        // columns of the sub-block that one warp owns and eliminates alone (one DMMA tile wide)
-constexpr size_t kGJAuxDoubles = kSub / kGJPanel + kSub;  // Gauss-Jordan bookkeeping: each panel's pivot rows as a mask; permutation and inverse
+constexpr int kGJNextLd = kGJPanel + 2;  // row stride of the next panel's buffer (16-byte rows, conflict-free)
+// Gauss-Jordan scratch: each panel's pivot rows as a mask; permutation and inverse; the next panel
+constexpr size_t kGJAuxDoubles = kSub / kGJPanel + kSub + kSub * kGJNextLd;
 constexpr size_t kPivotAuxBytes = (size_t(kSub) * kSmallLd + kGJAuxDoubles) * sizeof(double);
 constexpr size_t kPivotSmemBytes = size_t(kBlock) * kPivotLd * sizeof(double) + kPivotAuxBytes;
 constexpr size_t kUpdateSmemBytes = kUpdTileSmemBytes + 16;  // + the broadcast slot of the tile queue  // stages + C tile; the pivot aux reuses the stages
@@ -97,11 +99,12 @@ __device__ __forceinline__ double gj_reciprocal(double a) {
   return fma(y, fma(e, e, e), y);
 }
 
-// Eliminate the panel of columns j0 .. j0 + 7 of S by one warp (exchange steps inside the panel only).  Lane l holds
+// Eliminate the panel that becomes columns j0 .. j0 + 7 of S by one warp (exchange steps inside the panel only); src: the
+// panel's values (row stride src_ld).  Lane l holds
 // rows l and, where D = 64, l + 32; rows in `rows_before` have been pivots (or do not take part).  Returns the panel's pivot rows as
 // a mask; prow[0..7] gets them in order.
 template <int Ld, int D>
-__device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* prow, int j0, unsigned long long rows_before, bool& singular) {
+__device__ __forceinline__ unsigned long long gj_factor_panel(const double* src, int src_ld, double* S, int* prow, int j0, unsigned long long rows_before, bool& singular) {
   const int lane = threadIdx.x & 31;
   // rank of a row: its magnitude's leading 24 bits, then its index (the smaller row wins); 0 for a used row
   constexpr unsigned kRankMask = ~127u;
@@ -110,7 +113,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
   double v0[kGJPanel], v1[kGJPanel];
 #pragma unroll
   for (int i = 0; i < kGJPanel; i += 2) {
-    const double2 x = *reinterpret_cast<const double2*>(S + lane * Ld + j0 + i), y = *reinterpret_cast<const double2*>(S + (lane + D - 32) * Ld + j0 + i);
+    const double2 x = *reinterpret_cast<const double2*>(src + lane * src_ld + i), y = *reinterpret_cast<const double2*>(src + (lane + D - 32) * src_ld + i);
     v0[i] = x.x;
     v0[i + 1] = x.y;
     v1[i] = y.x;
@@ -125,16 +128,20 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
     const unsigned key = second ? h1 : h0;
     const unsigned best = __reduce_max_sync(0xffffffffu, key);
     constexpr unsigned kFirst = 1u << 21, kSpan = 0xffe00000u - kFirst;  // ranks of normal finite magnitudes
-    double c[kGJPanel];
-#pragma unroll
-    for (int i = 0; i < kGJPanel; ++i) c[i] = second ? v1[i] : v0[i];
-    const double inv_own = gj_reciprocal((key - kFirst) < kSpan ? c[0] : 1.0);  // of every lane's candidate, beside the search
+    const double inv_own = gj_reciprocal((key - kFirst) < kSpan ? (second ? v1[0] : v0[0]) : 1.0);  // of every lane's candidate, beside the search
     const int row = 127 - (int)(best & 127u);
+    const bool upper = D == 64 && row >= 32;  // the half that holds the pivot row: the same for all lanes
+    double p[kGJPanel];
+#pragma unroll
+    for (int i = 1; i < kGJPanel; ++i) p[i] = __shfl_sync(0xffffffffu, upper ? v1[i] : v0[i], row & 31);
+    const double inv = __shfl_sync(0xffffffffu, inv_own, row & 31);
     const bool own0 = row == lane, own1 = D == 64 && row == lane + 32;
     mask0 = own0 ? 0u : mask0;
     code0 = own0 ? 0u : code0;
     mask1 = own1 ? 0u : mask1;
     code1 = own1 ? 0u : code1;
+    singular |= !((best - kFirst) < kSpan);
+    if (lane == 0) prow[jj] = row;
     // the pivot row starts from zero with f = 1/a, every other row takes f = v/a
 #pragma unroll
     for (int i = 1; i < kGJPanel; ++i) {
@@ -143,12 +150,6 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
     }
     v0[0] = own0 ? 1.0 : v0[0];
     if (D == 64) v1[0] = own1 ? 1.0 : v1[0];
-    singular |= !((best - kFirst) < kSpan);
-    if (lane == 0) prow[jj] = row;
-    const double inv = __shfl_sync(0xffffffffu, inv_own, row & 31);
-    double p[kGJPanel];
-#pragma unroll
-    for (int i = 1; i < kGJPanel; ++i) p[i] = __shfl_sync(0xffffffffu, c[i], row & 31);
     const double f0 = v0[0] * inv, f1 = v1[0] * inv;
 #pragma unroll
     for (int i = 0; i + 1 < kGJPanel; ++i) {
@@ -174,11 +175,12 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(double* S, int* pr
 //
 // The exchange of one column is a serial chain (rank the rows, reciprocal, publish the row, update), so the work around
 // that chain is what costs.  It is blocked: one warp eliminates a panel of 8 columns in registers, with no barrier, no
-// shared memory and no branch inside the chain (295 cycles a column, issue-bound; 200 in a panel of 4 and 370 in one of
-// 16, while the step from one panel to the next takes 800 at any width).  The other columns take the 8 exchanges as
-// one rank-8 product on the FP64 tensor pipe: each warp keeps the 8-column strips that it owns in accumulator
-// registers, so that a panel costs one CTA barrier.  The owner of the next panel updates its strip alone, then
-// eliminates while the others update theirs.
+// shared memory and no branch inside the chain (240 cycles a column, issue-bound; 170 in a panel of 4 and 340 in one of
+// 16, while the step from one panel to the next costs the same at any width).  The other columns take the 8 exchanges as
+// one rank-8 product on the FP64 tensor pipe, each warp on the 8-column strip that it keeps in accumulator registers, so
+// that a panel costs one CTA barrier.  The strip that is the next panel is updated by four warps together (one on each
+// SM sub-partition, 4 tile products instead of 16 in the chain), from its place in S into a buffer; its owner
+// then eliminates it while the others update theirs.
 // Pivot choice: the largest magnitude by its leading 24 bits (13 of mantissa) among the unused rows, the smallest row
 // on ties; a NaN or an infinity ranks above all and is reported, as is a zero (or subnormal) pivot.
 // gauss_jordan_exchange leaves S in exchange form: inverse element (j, m) is S[perm[j] * Ld + iperm[m]] (j, m < n_act).
@@ -188,56 +190,65 @@ struct GJOrder {
 };
 template <int Ld, int kThreads, int D = kSub>
 __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& order, int n_act = D) {
-  constexpr int kWarps = kThreads / 32, kOwn = D / kGJPanel / kWarps;
+  static_assert(kThreads / 32 == D / kGJPanel, "a strip for every warp");
+  constexpr int kWarps = kThreads / 32, kTiles = D / 8 / 4;  // row tiles of the next panel that each of its four warps updates
   unsigned long long* panel_rows = reinterpret_cast<unsigned long long*>(aux);  // [kSub / kGJPanel]
   int* perm = reinterpret_cast<int*>(aux + kSub / kGJPanel);
   int* iperm = perm + kSub;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  double* panel = aux + kSub / kGJPanel + kSub;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, mr = lane >> 2, kr = lane & 3;
   bool singular = false;
   const int panels = n_act / kGJPanel;
   unsigned long long used = n_act == 64 ? 0ull : ~0ull << n_act;  // rows of all panels so far
-  GJStrip<D> g[kOwn];
-#pragma unroll
-  for (int o = 0; o < kOwn; ++o) gj_load_strip<Ld, D>(g[o], S, kGJPanel * (warp + o * kWarps));
+  GJStrip<D> g;
+  gj_load_strip<Ld, D>(g, S, kGJPanel * warp);
   __syncwarp();
+  if (warp == 0) {
+    const unsigned long long m = gj_factor_panel<Ld, D>(S, Ld, S, perm, 0, used, singular);
+    if (lane == 0) panel_rows[0] = m;
+  }
 #pragma unroll 1
-  for (int q = -1; q < panels; ++q) {
+  for (int q = 0; q < panels; ++q) {
     const int j0 = kGJPanel * q, next = q + 1;
-    unsigned long long mask = 0;
-    if (q >= 0) {
-      __syncthreads();  // panel q is in S; the updates of panel q - 1 are done
-      mask = panel_rows[q];
-      used |= mask;
-    }
-    const bool more = q + 1 < panels, mine = more && next % kWarps == warp;
-    if (mine) {  // the strip of the next panel first
-      if (q >= 0) {
+    __syncthreads();  // panel q is in S; the updates of panel q - 1 are done
+    const unsigned long long mask = panel_rows[q];
+    used |= mask;
+    if (next < panels) {
+      const int part = (warp - next) & (kWarps - 1);
+      if (part < 4) {
+        const double* c = S + kGJPanel * next;
+        const double w0 = -c[perm[j0 + kr] * Ld + mr], w1 = -c[perm[j0 + 4 + kr] * Ld + mr];
 #pragma unroll
-        for (int o = 0; o < kOwn; ++o)
-          if (next == warp + o * kWarps) {
-            gj_update_strip<Ld, D>(g[o], S, perm + j0, kGJPanel * next, j0, mask);
-            gj_store_strip<Ld, D>(g[o], S, kGJPanel * next);
-          }
-        asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
-        __syncwarp();
+        for (int i = 0; i < kTiles; ++i) {
+          const int row = 8 * (kTiles * part + i) + mr;
+          const bool pivot = (mask >> row) & 1ull;
+          const double2 old = *reinterpret_cast<const double2*>(c + row * Ld + 2 * kr);
+          double acc[2] = {pivot ? 0.0 : old.x, pivot ? 0.0 : old.y};
+          dmma_8x8x4(acc, S[row * Ld + j0 + kr], w0);
+          dmma_8x8x4(acc, S[row * Ld + j0 + 4 + kr], w1);
+          *reinterpret_cast<double2*>(panel + row * kGJNextLd + 2 * kr) = make_double2(acc[0], acc[1]);
+        }
+        if (part == 0) {
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          const unsigned long long m = gj_factor_panel<Ld, D>(panel, kGJNextLd, S, perm + kGJPanel * next, kGJPanel * next, used, singular);
+          if (lane == 0) panel_rows[next] = m;
+        } else {
+          asm volatile("bar.arrive 1, 128;" ::: "memory");
+        }
       }
-      const unsigned long long m = gj_factor_panel<Ld, D>(S, perm + j0 + kGJPanel, j0 + kGJPanel, used, singular);
-      if (lane == 0) panel_rows[q + 1] = m;
-    } else if (more && q >= 0) {
-      asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");  // the next panel's owner has the tensor pipe to itself
     }
-    if (q < 0) continue;
-#pragma unroll
-    for (int o = 0; o < kOwn; ++o) {
-      const int strip = warp + o * kWarps;
-      if (strip == q) gj_load_strip<Ld, D>(g[o], S, j0);
-      else if (strip < panels && !(mine && strip == next)) gj_update_strip<Ld, D>(g[o], S, perm + j0, kGJPanel * strip, j0, mask);
+    if (warp == q) {
+      gj_load_strip<Ld, D>(g, S, j0);
+    } else if (warp < panels && warp != next) {
+      gj_update_strip<Ld, D>(g, S, perm + j0, kGJPanel * warp, j0, mask);
+      if (warp == next + 1) {  // the panel after the next: to its place
+        __syncwarp();
+        gj_store_strip<Ld, D>(g, S, kGJPanel * warp);
+      }
     }
   }
   __syncthreads();  // the last panel's E has been read
-#pragma unroll
-  for (int o = 0; o < kOwn; ++o)
-    if (warp + o * kWarps < panels) gj_store_strip<Ld, D>(g[o], S, kGJPanel * (warp + o * kWarps));
+  if (warp < panels) gj_store_strip<Ld, D>(g, S, kGJPanel * warp);
   if (t < n_act) iperm[perm[t]] = t;
   order.perm = perm;
   order.iperm = iperm;

@@ -16,7 +16,7 @@
 // Flags (per matrix, monotonic over the sweeps of one call, so that only the first one clears them): per lower tile the number
 // of steps applied, per block row the last panel, the last inverted pivot, per step the finished updates (a
 // panel slot is rewritten kFineSlots steps later, once its readers are done).
-// A step of the chain takes 24-25 us: 15 for the block's inversion, 2.3 for each of its two products (one SM's FP64 pipe),
+// A step of the chain takes 22-23 us: 13 for the block's inversion, 2.3 and 1.3 for its two products (one SM's FP64 pipe),
 // 2 for publishing P^{-1}, the rest the flag's way to the next CTA, its load of P^{-1} and the stores in between.
 #pragma once
 
@@ -129,6 +129,48 @@ __device__ __forceinline__ void fine_product(FineAcc& acc, const double* A, int 
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int w = 0; w < 4; ++w) dmma_8x8x4(acc.v[u][w], a[u], b[w]);
+  }
+}
+// S[r][c] = S[c][r] = old - (A B^T)[r][c] for the lower triangle, A, B and S 64 x 64 with row stride kSmallLd.  Of the 36 lower 8 x 8
+// tiles warp s < 4 multiplies tile row s and warp 4 + s tile row 7 - s: nine for every SM sub-partition, where the whole
+// square takes sixteen.  A template of the tile row, since predicated-off multiplications cost as much as real ones.
+// old: the row's tiles from C (row stride ld).
+template <int kRow>
+__device__ __forceinline__ void fine_lower_row(const double* A, const double* B, double* S, const double* C, long long ld) {
+  const int lane = threadIdx.x & 31, mr = lane >> 2, kr = lane & 3, r = 8 * kRow + mr;
+  double2 old[kRow + 1];
+  double acc[kRow + 1][2];
+#pragma unroll
+  for (int i = 0; i <= kRow; ++i) {
+    old[i] = __ldcg(reinterpret_cast<const double2*>(C + (long long)r * ld + 8 * i + 2 * kr));
+    acc[i][0] = acc[i][1] = 0.0;
+  }
+  const double *a = A + r * kSmallLd + kr, *b = B + mr * kSmallLd + kr;
+#pragma unroll 2
+  for (int k = 0; k < kSub; k += 4) {
+    const double x = a[k];
+#pragma unroll
+    for (int i = 0; i <= kRow; ++i) dmma_8x8x4(acc[i], x, b[8 * i * kSmallLd + k]);
+  }
+  __syncthreads();  // S may be A
+#pragma unroll
+  for (int i = 0; i <= kRow; ++i) {
+    const int c = 8 * i + 2 * kr;
+    const double x = old[i].x - acc[i][0], y = old[i].y - acc[i][1];
+    if (i < kRow || r >= c) S[r * kSmallLd + c] = S[c * kSmallLd + r] = x;
+    if (i < kRow || r >= c + 1) S[r * kSmallLd + c + 1] = S[(c + 1) * kSmallLd + r] = y;
+  }
+}
+__device__ __forceinline__ void fine_lower_update(const double* A, const double* B, double* S, const double* C, long long ld) {
+  switch (threadIdx.x >> 5) {
+    case 0: fine_lower_row<0>(A, B, S, C, ld); break;
+    case 1: fine_lower_row<1>(A, B, S, C, ld); break;
+    case 2: fine_lower_row<2>(A, B, S, C, ld); break;
+    case 3: fine_lower_row<3>(A, B, S, C, ld); break;
+    case 4: fine_lower_row<7>(A, B, S, C, ld); break;
+    case 5: fine_lower_row<6>(A, B, S, C, ld); break;
+    case 6: fine_lower_row<5>(A, B, S, C, ld); break;
+    default: fine_lower_row<4>(A, B, S, C, ld); break;
   }
 }
 __device__ __forceinline__ void fine_zero(FineAcc& acc) {
@@ -276,15 +318,6 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       if (!fine_wait(w, fine_need(mine, now, diagonal, now, readers, readers_target, mine, now), b, slot + 1)) return;
       for (int half = 0; half < 2; ++half) fine_stage(SA, T, w.ld, half);
       cp_async_commit();
-      FineAcc old;
-      if (chain) {
-        const double* C = Mb + (long long)j * kSub * w.ld + j * kSub;
-        fine_each(old, [&](int r, int c, double(&d)[2]) {
-          const double2 x = __ldcg(reinterpret_cast<const double2*>(C + (long long)r * w.ld + c));
-          d[0] = x.x;
-          d[1] = x.y;
-        });
-      }
       cp_async_wait<0>();
       __syncthreads();
 #pragma unroll 4
@@ -323,14 +356,7 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       }
       if (!chain) continue;
       // M(j, j) - X R^T (here j = k + 1 > k: X[c][k], R[c][k]), lower half, mirrored
-      fine_zero(acc);
-      fine_product(acc, SA, kSmallLd, 1, SC, 1, kSmallLd, 0, kSub);
-      __syncthreads();
-      fine_sub(old, acc);
-      fine_each(old, [&](int r, int c, double(&d)[2]) {
-        if (r >= c) SA[r * kSmallLd + c] = SA[c * kSmallLd + r] = d[0];
-        if (r >= c + 1) SA[r * kSmallLd + c + 1] = SA[(c + 1) * kSmallLd + r] = d[1];
-      });
+      fine_lower_update(SA, SC, SA, Mb + (long long)j * kSub * w.ld + j * kSub, w.ld);
       __syncthreads();
       if (tid == kFineThreads - 64) atomicAdd(done + k, 1);
       fine_invert(w, b, j, SA, SC, aux, Mb, f + 2 * nt, const_cast<int*>(ver) + fine_lower(j, j), now + 2);
@@ -451,10 +477,10 @@ inline cudaError_t sweep_any(FineState& fine, double* M, long long mstride, int 
 
 // Whether a batch of FP64 sweeps of n_used rows takes the 64-tile path: where its estimated time is below that of the
 // 128-tile steps, both the larger of a latency (per step of the chain) and a throughput (per cubed tile count) term, in
-// us.  Measured, us a sweep, 128-tile steps / here: N = 192, batch 16: 221 / 86; N = 231, batch 16: 221 / 113, batch 128: 241 / 207;
-// N = 396, batch 8: 442 / 190; N = 512, batch 32: 484 / 334, batch 64: 622 / 672; N = 660, batch 4: 664 / 293, batch 64: 1728 / 1688;
-// N = 1024, batch 8: 925 / 605, batch 16: 1157 / 1206; N = 1984, batch 1: 1772 / 809, batch 8: 3524 / 4230; N = 100 (one
-// 128 block, no steps): 52 / 61.
+// us.  Measured, us a sweep, 128-tile steps / here: N = 192, batch 16: 221 / 76; N = 231, batch 16: 221 / 98, batch 128: 241 / 207;
+// N = 396, batch 8: 442 / 166; N = 512, batch 32: 484 / 324, batch 64: 622 / 672; N = 660, batch 4: 664 / 255, batch 64: 1728 / 1688;
+// N = 1024, batch 8: 925 / 594, batch 16: 1157 / 1206; N = 1984, batch 1: 1772 / 760, batch 8: 3524 / 4230; N = 100 (one
+// 128 block, no steps): 50 / 53.
 inline bool use_fine(int n_used, size_t batch) {
   const int nt = fine_tiles(n_used), steps = (n_used + kBlock - 1) / kBlock;
   if (steps < 2 || nt > kFineMaxTiles) return false;
