@@ -46,25 +46,33 @@ __device__ __forceinline__ void stage_rows(double* dst, const double* src, long 
   }
 }
 
-template <int kC = kChunk>
-__device__ __forceinline__ void mma_chunk(TileAcc& acc, const double* As, const double* Bs, int warp, int lane) {
-  const int wm = (warp >> 2) * 64;
-  const int wn = (warp & 3) * 32;
-  const int kr = lane & 3;
-  const int mr = lane >> 2;
+// Multiply a chunk of kC rows.  `then` (the next chunk's copies) runs once the first rows' products have been issued, so
+// that its address arithmetic and the wait for the first fragments do not both leave the tensor pipe idle behind the chunk's
+// barrier; the next rows' fragments are loaded ahead of the products in hand.
+struct MmaFragments {
+  double a[8], b[4];
+};
+__device__ __forceinline__ void load_fragments(MmaFragments& f, const double* arow, const double* brow) {
+#pragma unroll
+  for (int mt = 0; mt < 8; ++mt) f.a[mt] = arow[mt * 8];
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) f.b[nt] = brow[nt * 8];
+}
+template <int kC = kChunk, class F>
+__device__ __forceinline__ void mma_chunk(TileAcc& acc, const double* As, const double* Bs, int warp, int lane, F&& then) {
+  const double* arow = As + (lane & 3) * kStride + (warp >> 2) * 64 + (lane >> 2);
+  const double* brow = Bs + (lane & 3) * kStride + (warp & 3) * 32 + (lane >> 2);
+  MmaFragments f[2];
+  load_fragments(f[0], arow, brow);
 #pragma unroll
   for (int kk = 0; kk < kC; kk += 4) {
-    double a[8], b[4];
-    const double* arow = As + (kk + kr) * kStride + wm + mr;
-    const double* brow = Bs + (kk + kr) * kStride + wn + mr;
-#pragma unroll
-    for (int mt = 0; mt < 8; ++mt) a[mt] = arow[mt * 8];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) b[nt] = brow[nt * 8];
+    const MmaFragments& now = f[(kk / 4) & 1];
+    if (kk + 4 < kC) load_fragments(f[(kk / 4 + 1) & 1], arow + (kk + 4) * kStride, brow + (kk + 4) * kStride);
 #pragma unroll
     for (int mt = 0; mt < 8; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) dmma_8x8x4(acc.v[mt][nt], a[mt], b[nt]);
+      for (int nt = 0; nt < 4; ++nt) dmma_8x8x4(acc.v[mt][nt], now.a[mt], now.b[nt]);
+    if (kk == 0) then();
   }
 }
 
@@ -91,21 +99,21 @@ __device__ inline void tile_gemm_tn(TileAcc& acc, const double* A, long long lda
     cp_async_commit();
   }
   for (int c = 0; c < nchunks; ++c) {
-    if (c + 1 < nchunks) {
-      double* next = smem + ((c + 1) & 1) * kStage;
-      const int k = row_of(c + 1);
-      stage_rows(next, A, lda, k, tid);
-      stage_rows(next + kChunk * kStride, B, ldb, k, tid);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    // one barrier a chunk: behind it chunk c is there for every thread and the other stage's readers are done
+    cp_async_wait<0>();
     __syncthreads();
     const double* cur = smem + (c & 1) * kStage;
-    mma_chunk(acc, cur, cur + kChunk * kStride, warp, lane);
-    __syncthreads();
+    mma_chunk(acc, cur, cur + kChunk * kStride, warp, lane, [&] {
+      if (c + 1 < nchunks) {
+        double* next = smem + ((c + 1) & 1) * kStage;
+        const int k = row_of(c + 1);
+        stage_rows(next, A, lda, k, tid);
+        stage_rows(next + kChunk * kStride, B, ldb, k, tid);
+        cp_async_commit();
+      }
+    });
   }
+  __syncthreads();
 }
 
 // Write the accumulator into a [128][kStride] shared tile: Cs[row][col] = scale * acc.
@@ -289,8 +297,15 @@ constexpr int kUpdStageDoubles64 = 2 * 2 * kUpdChunk * kStride;  // FP64 stages:
 constexpr int kUpdStageDoubles = kUpdStageDoubles64 > kSplitStageWords ? kUpdStageDoubles64 : kSplitStageWords;  // 2 split stages = 8704 doubles
 constexpr size_t kUpdTileSmemBytes = (size_t(kUpdStageDoubles) + size_t(kBlock) * kStride) * sizeof(double);  // 204800
 
-__device__ __forceinline__ void mma_chunk_any(TileAcc& acc, const double* As, const double* Bs, int warp, int lane) { mma_chunk<kUpdChunk>(acc, As, Bs, warp, lane); }
-__device__ __forceinline__ void mma_chunk_any(TileAcc32& acc, const double* As, const double* Bs, int warp, int lane) { mma_chunk_tf32x3<kUpdChunk>(acc, As, Bs, warp, lane); }
+template <class F>
+__device__ __forceinline__ void mma_chunk_any(TileAcc& acc, const double* As, const double* Bs, int warp, int lane, F&& then) {
+  mma_chunk<kUpdChunk>(acc, As, Bs, warp, lane, then);
+}
+template <class F>
+__device__ __forceinline__ void mma_chunk_any(TileAcc32& acc, const double* As, const double* Bs, int warp, int lane, F&& then) {
+  then();
+  mma_chunk_tf32x3<kUpdChunk>(acc, As, Bs, warp, lane);
+}
 __device__ __forceinline__ void acc_zero(TileAcc& acc) {
 #pragma unroll
   for (int mt = 0; mt < 8; ++mt)
@@ -306,15 +321,18 @@ __device__ __forceinline__ void acc_zero(TileAcc32& acc) {
       for (int q = 0; q < 4; ++q) acc.v[mt][nt][q] = 0.0f;
 }
 
-// The product is split so that a persistent CTA can start the next tile's loads early:
-// issue_update_chunk0 and issue_update_ctile each commit one cp.async group, and
-// update_mainloop expects exactly that order of groups in flight (chunk 0, C tile) and
-// then commits chunks 1 .. K/kUpdChunk - 1 itself.
-__device__ __forceinline__ void issue_update_chunk0(const double* A, long long lda, const double* B, long long ldb, double* stages) {
+// The product is split so that a persistent CTA can start the next tile's loads early: issue_update_chunks (chunks 0 and
+// 1, one cp.async group each) and issue_update_ctile (one group) are issued in that order, and update_mainloop expects
+// exactly those groups in flight and then commits chunks 2 .. K/kUpdChunk - 1 itself.
+__device__ __forceinline__ void issue_update_chunks(const double* A, long long lda, const double* B, long long ldb, double* stages) {
   const int tid = threadIdx.x;
-  stage_rows<kUpdChunk>(stages, A, lda, 0, tid);
-  stage_rows<kUpdChunk>(stages + kUpdChunk * kStride, B, ldb, 0, tid);
-  cp_async_commit();
+  constexpr int kStage = 2 * kUpdChunk * kStride;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    stage_rows<kUpdChunk>(stages + c * kStage, A, lda, c * kUpdChunk, tid);
+    stage_rows<kUpdChunk>(stages + c * kStage + kUpdChunk * kStride, B, ldb, c * kUpdChunk, tid);
+    cp_async_commit();
+  }
 }
 __device__ __forceinline__ void issue_update_ctile(double* Cs, const double* Cg, long long ldc) {
   const int tid = threadIdx.x;
@@ -326,8 +344,8 @@ __device__ __forceinline__ void issue_update_ctile(double* Cs, const double* Cg,
   cp_async_commit();
 }
 
-// acc = sum_{k < K} A[k][.]^T B[k][.] (K a multiple of kUpdChunk, at least 2 chunks), with
-// chunk 0 and the C tile already issued.  On return Cs holds C and the staging region is
+// acc = sum_{k < K} A[k][.]^T B[k][.] (K a multiple of kUpdChunk, at least 3 chunks), with
+// chunks 0, 1 and the C tile already issued.  On return Cs holds C and the staging region is
 // free (ends with a __syncthreads()).
 template <class Acc>
 __device__ inline void update_mainloop(Acc& acc, const double* A, long long lda, const double* B, long long ldb, int K, double* stages) {
@@ -338,32 +356,28 @@ __device__ inline void update_mainloop(Acc& acc, const double* A, long long lda,
   constexpr int kStage = 2 * kUpdChunk * kStride;
   const int nchunks = K / kUpdChunk;
   for (int c = 0; c < nchunks; ++c) {
-    if (c + 1 < nchunks) {
-      double* next = stages + ((c + 1) & 1) * kStage;
-      stage_rows<kUpdChunk>(next, A, lda, (c + 1) * kUpdChunk, tid);
-      stage_rows<kUpdChunk>(next + kUpdChunk * kStride, B, ldb, (c + 1) * kUpdChunk, tid);
-      cp_async_commit();
-    }
-    // groups newer than chunk c that may stay in flight: c = 0 -> C tile and chunk 1;
-    // later -> chunk c + 1 only; the last chunk waits for everything
-    if (c + 1 >= nchunks) {
-      cp_async_wait<0>();
-    } else if (c == 0) {
-      cp_async_wait<2>();
-    } else {
-      cp_async_wait<1>();
-    }
-    __syncthreads();
+    // chunk c has landed; newer groups that may stay in flight: chunk 1 and the C tile, then the C tile, then none
+    if (c == 0) cp_async_wait<2>();
+    else if (c == 1) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();  // for every thread; and the other stage's readers (chunk c - 1) are done
     const double* cur = stages + (c & 1) * kStage;
-    mma_chunk_any(acc, cur, cur + kUpdChunk * kStride, warp, lane);
-    __syncthreads();
+    mma_chunk_any(acc, cur, cur + kUpdChunk * kStride, warp, lane, [&] {
+      if (c >= 1 && c + 1 < nchunks) {
+        double* next = stages + ((c + 1) & 1) * kStage;
+        stage_rows<kUpdChunk>(next, A, lda, (c + 1) * kUpdChunk, tid);
+        stage_rows<kUpdChunk>(next + kUpdChunk * kStride, B, ldb, (c + 1) * kUpdChunk, tid);
+        cp_async_commit();
+      }
+    });
   }
+  __syncthreads();
 }
 
 // The whole product in one call: Cs <- C tile while acc = A^T B.
 template <class Acc>
 __device__ inline void tile_update_product(Acc& acc, const double* A, long long lda, const double* B, long long ldb, int K, double* stages, double* Cs, const double* Cg, long long ldc) {
-  issue_update_chunk0(A, lda, B, ldb, stages);
+  issue_update_chunks(A, lda, B, ldb, stages);
   issue_update_ctile(Cs, Cg, ldc);
   update_mainloop(acc, A, lda, B, ldb, K, stages);
 }

@@ -605,7 +605,7 @@ __device__ __forceinline__ void update_tile_of(int g, int per, int t, int kb, in
 }
 
 // Persistent tile loop of the trailing update: tiles come from the step's atomic queue; the
-// next tile's first K-chunk is issued before the current tile's epilogue and its C tile
+// next tile's first two K-chunks are issued before the current tile's epilogue and its C tile
 // right after, so only the product itself is on the critical path of a CTA.
 template <bool kSym, class Acc>
 __device__ inline void update_tiles(double* M, long long mstride, int ld, int kb, const double* cold, long long cstride, int t, int per, int total, bool skip_pivot, int* queue,
@@ -635,7 +635,7 @@ __device__ inline void update_tiles(double* M, long long mstride, int ld, int kb
   if (g >= total) return;
   int b, ta, tb;
   update_tile_of<kSym>(g, per, t, kb, b, ta, tb);
-  issue_update_chunk0(cold + (long long)b * cstride + ta * kBlock, ld, M + (long long)b * mstride + (long long)k0 * ld + tb * kBlock, ld, smem);
+  issue_update_chunks(cold + (long long)b * cstride + ta * kBlock, ld, M + (long long)b * mstride + (long long)k0 * ld + tb * kBlock, ld, smem);
   issue_update_ctile(Cs, M + (long long)b * mstride + (long long)ta * kBlock * ld + tb * kBlock, ld);
   for (;;) {
     double* Mb = M + (long long)b * mstride;
@@ -646,7 +646,7 @@ __device__ inline void update_tiles(double* M, long long mstride, int ld, int kb
     int bn = 0, tan = 0, tbn = 0;
     if (gn < total) {
       update_tile_of<kSym>(gn, per, t, kb, bn, tan, tbn);
-      issue_update_chunk0(cold + (long long)bn * cstride + tan * kBlock, ld, M + (long long)bn * mstride + (long long)k0 * ld + tbn * kBlock, ld, smem);
+      issue_update_chunks(cold + (long long)bn * cstride + tan * kBlock, ld, M + (long long)bn * mstride + (long long)k0 * ld + tbn * kBlock, ld, smem);
     }
     // C - acc straight from registers (with the transpose of an off-diagonal tile of the
     // symmetric sweep, a diagonal tile symmetrised from its lower half); Cs is free after
