@@ -71,7 +71,9 @@ size_t ldmd_layout(ticc::LdmdLayout& L, int n, int n_energy, int n_block, int n_
   const int used = is_complex ? 2 * n : n;
   const size_t q_chunk = std::min((size_t)n_sector * n_block, L.scratch_doubles / ticc::sweep_scratch_doubles(L.npr));
   const bool fine_m = precision == TICC_PRECISION_FP64 && ticc::use_fine(used, batch), fine_q = ticc::use_fine(n, q_chunk);
-  const size_t fine = std::max(fine_m ? ticc::fine_total_doubles(ticc::fine_tiles(used), batch) : 0, fine_q ? ticc::fine_total_doubles(ticc::fine_tiles(n), q_chunk) : 0);
+  const size_t q_count = (size_t)n_sector * n_block;
+  L.joint_q = ticc::ldmd_joint_qmid(n, batch, q_count, is_complex, precision == TICC_PRECISION_FP64);
+  const size_t fine = std::max(fine_m ? ticc::fine_total_doubles(ticc::fine_tiles(used), batch + (L.joint_q ? q_count : 0)) : 0, fine_q ? ticc::fine_total_doubles(ticc::fine_tiles(n), q_chunk) : 0);
   double* fine_base = fine > 0 ? c.take<double>(fine) : nullptr;
   L.fine = fine_m ? fine_base : nullptr;
   L.fine_q = fine_q ? fine_base : nullptr;

@@ -47,6 +47,7 @@ struct LdmdLayout {
   int* reduced;   // [n_sector] leading sweep blocks taken in TF32x3 (mixed mode), else null
   double* fine;   // 64-tile sweeps' panels and flags (FP64 work matrices where they fit), else null
   double* fine_q; // the same region for the Q_mid sweeps, else null
+  bool joint_q;   // the region holds the first work matrices and all Q_mid matrices together
   float* split;   // FP32 operand panels of the reduced steps' tcgen05 update (mixed mode), else null
 };
 
@@ -590,12 +591,14 @@ inline unsigned grid_for(long long work, int threads, unsigned cap = 1u << 16) {
   return (unsigned)(blocks > cap ? cap : blocks);
 }
 
-// Q_mid for every (sector, block) of the call (batched sweep, chunked to fit scratch).
-inline cudaError_t ldmd_qmid(const LdmdSectors& sec, LdmdLayout& L, int* status, cudaStream_t stream) {
+// Q_mid for every (sector, block) of the call: build, sweep (batched, chunked to fit scratch) and finish.
+inline void ldmd_qmid_build(const LdmdSectors& sec, const LdmdLayout& L, cudaStream_t stream) {
+  ldmd_qmid_build_kernel<<<dim3(grid_for((long long)L.npr * L.npr, 256, 4096), sec.n_sector * L.n_block), 256, 0, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm);
+  note_launch();
+}
+inline cudaError_t ldmd_qmid_sweep(const LdmdSectors& sec, const LdmdLayout& L, int* status, cudaStream_t stream) {
   const long long per = (long long)L.npr * L.npr;
   const int count = sec.n_sector * L.n_block;
-  ldmd_qmid_build_kernel<<<dim3(grid_for(per, 256, 4096), count), 256, 0, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm);
-  note_launch();
   const int chunk = (int)(L.scratch_doubles / sweep_scratch_doubles(L.npr));
   FineState fine{L.fine_q};
   for (int s0 = 0; s0 < count; s0 += chunk) {
@@ -603,10 +606,17 @@ inline cudaError_t ldmd_qmid(const LdmdSectors& sec, LdmdLayout& L, int* status,
     cudaError_t e = sweep_any(fine, L.Qm + (long long)s0 * per, per, L.npr, cnt, L.scratch, status, stream, nullptr, L.n, nullptr);
     if (e != cudaSuccess) return e;
   }
-  ldmd_qmid_finish_kernel<<<dim3(grid_for(per, 256, 4096), count), 256, 0, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm);
+  return cudaSuccess;
+}
+inline cudaError_t ldmd_qmid_finish(const LdmdSectors& sec, const LdmdLayout& L, cudaStream_t stream) {
+  ldmd_qmid_finish_kernel<<<dim3(grid_for((long long)L.npr * L.npr, 256, 4096), sec.n_sector * L.n_block), 256, 0, stream>>>(sec, L.n, L.n_block, L.npr, L.Qm);
   note_launch();
   return cudaGetLastError();
 }
+
+// Whether the Q_mid matrices of a call are swept beside its first work matrices, in one launch: they have the same size
+// in a real call, and the 64-tile sweep is bound by its chain, which more matrices do not lengthen.
+inline bool ldmd_joint_qmid(int n, size_t batch, size_t q_count, int is_complex, bool fp64) { return fp64 && !is_complex && q_count <= 64 && use_fine(n, batch) && use_fine(n, batch + q_count); }
 
 template <int D>
 inline cudaError_t ldmd_small_qmid(const LdmdSectors& sec, const LdmdLayout& L, int* status, cudaStream_t stream) {
@@ -642,7 +652,11 @@ inline cudaError_t ldmd_propagate(double* Y, const double* energies, double mu, 
     if (e != cudaSuccess) return e;
     return rows <= 32 ? ldmd_small<32>(Y, sec, L, status, stream) : rows <= 64 ? ldmd_small<64>(Y, sec, L, status, stream) : ldmd_small<128>(Y, sec, L, status, stream);
   }
-  cudaError_t err = ldmd_qmid(sec, L, status, stream);
+  // one launch sweeps the first sector's work matrices and every Q_mid where the layout has room for both
+  const bool joint = L.joint_q;
+  ldmd_qmid_build(sec, L, stream);
+  cudaError_t err = joint ? cudaSuccess : ldmd_qmid_sweep(sec, L, status, stream);
+  if (err == cudaSuccess && !joint) err = ldmd_qmid_finish(sec, L, stream);
   if (err != cudaSuccess) return err;
   const long long mstride = (long long)L.np * L.np;
   const int used = L.is_complex ? 2 * L.n : L.n;  // rows of the work matrix beyond these are identity padding
@@ -650,7 +664,12 @@ inline cudaError_t ldmd_propagate(double* Y, const double* energies, double mu, 
   for (int s = 0; s < sec.n_sector; ++s) {
     err = ldmd_elementwise(s == 0 ? 0 : 1, s, sec, L, Y, Y, stream);
     if (err != cudaSuccess) return err;
-    err = sweep_any(fine, L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
+    if (s == 0 && joint) {
+      err = fine_sweep(fine, L.M, mstride, L.np, used, batch, status, stream, L.Qm, (long long)L.npr * L.npr, sec.n_sector * L.n_block);
+      if (err == cudaSuccess) err = ldmd_qmid_finish(sec, L, stream);
+    } else {
+      err = sweep_any(fine, L.M, mstride, L.np, batch, L.scratch, status, stream, L.reduced ? L.reduced + s : nullptr, used, L.split);
+    }
     if (err != cudaSuccess) return err;
     err = ldmd_elementwise(2, s, sec, L, Y, Y, stream);
     if (err != cudaSuccess) return err;

@@ -46,6 +46,9 @@ struct FineSweep {
   double* M;
   long long mstride;
   int ld, nt, batch;
+  double* M2;      // matrices `split` .. batch - 1 (same size and row stride) lie here
+  long long mstride2;
+  int split;
   double* slots;   // [batch][kFineSlots][2 (X, R)][nt][64][64]
   double* pinv;    // [batch][kFinePinv][64][64]
   int* flags;      // [batch][fine_flag_ints(nt)]
@@ -55,6 +58,8 @@ struct FineSweep {
   int sweep;       // number of this sweep in the call (the finished-update counters grow by one sweep's worth each)
   int queue_base;  // queue value at which this launch starts
 };
+
+__device__ __forceinline__ double* fine_matrix(const FineSweep& w, int b) { return b < w.split ? w.M + (long long)b * w.mstride : w.M2 + (long long)(b - w.split) * w.mstride2; }
 
 // Positions 0 .. nt - 2 of the block rows other than k, from k + 1 on, cyclic.
 __device__ __forceinline__ int fine_row_at(int k, int nt, int pos) {
@@ -254,7 +259,7 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
     __syncthreads();  // also: the previous unit's shared memory is free
     if (u < 0 || u >= total) return;
     if (u < batch) {  // the first pivot
-      double* Mb = w.M + (long long)u * w.mstride;
+      double* Mb = fine_matrix(w, u);
       for (int half = 0; half < 2; ++half) fine_stage(SA, Mb, w.ld, half);
       cp_async_commit();
       cp_async_wait<0>();
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
         }
       }
     }
-    double* Mb = w.M + (long long)b * w.mstride;
+    double* Mb = fine_matrix(w, b);
     int* f = w.flags + (long long)b * fints;
     int* done = f + nt;
     const int* ver = f + 2 * nt + 2;
@@ -421,7 +426,9 @@ struct FineState {
   int nt = 0, batch = 0, sweeps = 0, queue = 0;
 };
 
-inline cudaError_t fine_sweep(FineState& state, double* M, long long mstride, int ld, int n_used, int batch, int* status, cudaStream_t stream) {
+// M2 (optional): `batch2` more matrices of the same size, swept in the same launch.
+inline cudaError_t fine_sweep(FineState& state, double* M, long long mstride, int ld, int n_used, int batch, int* status, cudaStream_t stream, double* M2 = nullptr, long long mstride2 = 0,
+                              int batch2 = 0) {
   cudaError_t e = cudaFuncSetAttribute(sweep_fine_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFineSmemBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fine_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFineSmemBytes);
   if (e != cudaSuccess) return e;
@@ -433,6 +440,10 @@ inline cudaError_t fine_sweep(FineState& state, double* M, long long mstride, in
   FineSweep w{};
   w.M = M;
   w.mstride = mstride;
+  w.M2 = M2;
+  w.mstride2 = mstride2;
+  w.split = batch;
+  batch += batch2;
   w.ld = ld;
   w.nt = nt;
   w.batch = batch;
