@@ -414,10 +414,10 @@ struct SmallShape {
   static constexpr int kPerSM = D == 32 ? 4 : D == 64 ? 2 : 1;
 };
 
-// Invert the matrix in S (used rows: `used`); get(r, c) of the functor passed on is then the swept value
-// -A^{-1}(r, c), symmetrised.  put(r, c, f) for every (r, c) < n_act replaces the matrix by f(r, c, swept value).
-template <int D, class F>
-__device__ inline bool small_sweep_then(double* S, double* aux, int used, F&& f) {
+// Invert the matrix in S (used rows: `used`) and call f(r, c, v, w) for every c <= r < used with the swept value v = -A^{-1}(r, c),
+// symmetrised, and w = pre(r, c): what f needs from global memory, fetched before the inversion where registers hold it.
+template <int D, class P, class F>
+__device__ inline bool small_sweep_then(double* S, double* aux, int used, P&& pre, F&& f) {
   using Sh = SmallShape<D>;
   const int n_act = (int)round_up(used, kGJPanel);
   if constexpr (D == 128) {
@@ -427,14 +427,19 @@ __device__ inline bool small_sweep_then(double* S, double* aux, int used, F&& f)
       const int r = e / D, c = e % D;
       if (c > r) continue;
       const double v = 0.5 * (S[r * Sh::kLd + c] + S[c * Sh::kLd + r]);
-      f(r, c, v);
+      f(r, c, v, pre(r, c));
     }
     __syncthreads();
     return singular;
   } else {
+    double w[Sh::kPer], x[Sh::kPer];
+#pragma unroll
+    for (int u = 0; u < Sh::kPer; ++u) {
+      const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;
+      w[u] = (D == 32 && r < used && c <= r) ? pre(r, c) : 0.0;  // (64 rows: the registers are the exchange's)
+    }
     GJOrder order;
     const bool singular = gauss_jordan_exchange<Sh::kLd, Sh::kThreads, D>(S, aux, order, n_act);
-    double x[Sh::kPer];
 #pragma unroll
     for (int u = 0; u < Sh::kPer; ++u) {
       const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;
@@ -445,7 +450,7 @@ __device__ inline bool small_sweep_then(double* S, double* aux, int used, F&& f)
 #pragma unroll
     for (int u = 0; u < Sh::kPer; ++u) {
       const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;
-      if (r < used && c <= r) f(r, c, x[u]);
+      if (r < used && c <= r) f(r, c, x[u], D == 32 ? w[u] : pre(r, c));
     }
     __syncthreads();
     return singular;
@@ -484,7 +489,7 @@ __global__ void __launch_bounds__(SmallShape<D>::kThreads, SmallShape<D>::kPerSM
     S[i * Sh::kLd + j] = (i == j) ? 1.0 : -h * h * sym(Wm, n, i, j) / 6.0;
   }
   __syncthreads();
-  const bool singular = small_sweep_then<D>(S, aux, n, [&](int i, int j, double v) {
+  const bool singular = small_sweep_then<D>(S, aux, n, [](int, int) { return 0.0; }, [&](int i, int j, double v, double) {
     const double q = 4.0 / h * (-v - (i == j ? 1.0 : 0.0));
     Q[(long long)i * npr + j] = q;
     Q[(long long)j * npr + i] = q;
@@ -505,31 +510,49 @@ __global__ void __launch_bounds__(SmallShape<D>::kThreads, SmallShape<D>::kPerSM
   bool singular = false;
   small_pad<D>(S, used);
   double* Yb = Y + (long long)b * n * n * (cplx ? 2 : 1);
+  const long long wb = g * sec.wb_stride;
+  double h_next = sec.h[0], h = 0.0, hp = 0.0, ref_next = 0.0, y1_next = 0.0, y2_next = 0.0;
+  const auto fetch = [&](int s) {  // a sector's channel values, a channel a thread, ahead of the sector
+    h_next = sec.h[s];
+    const int i = threadIdx.x;
+    if (i < n) {
+      ref_next = sec.Wm[s * sec.wm_stride + wb + (long long)i * n + i];
+      y1_next = L.y1[((long long)s * batch + b) * n + i];
+      y2_next = L.y2[((long long)s * batch + b) * n + i];
+    }
+  };
+  fetch(0);
   for (int s = 0; s < sec.n_sector; ++s) {
     double *ref = vec + 3 * D * (s & 1), *y1 = ref + D, *y2 = y1 + D;
     const double *refp = vec + 3 * D * ((s + 1) & 1), *y1p = refp + D, *y2p = y1p + D;
-    const double h = sec.h[s], hp = s > 0 ? sec.h[s - 1] : 0.0;
-    const long long wb = g * sec.wb_stride;
-    const double *Ws = sec.Ws + s * sec.ws_stride + wb, *Wm = sec.Wm + s * sec.wm_stride + wb;
+    hp = h;
+    h = h_next;
+    const double* Ws = sec.Ws + s * sec.ws_stride + wb;
     const double *We = sec.We + s * sec.we_stride + wb, *Wep = s > 0 ? sec.We + (s - 1) * sec.we_stride + wb : We;
     const double* Q = L.Qm + ((long long)s * L.n_block + g) * L.npr * L.npr;
-    for (int i = threadIdx.x; i < n; i += Sh::kThreads) {
-      ref[i] = Wm[(long long)i * n + i];
-      y1[i] = L.y1[((long long)s * batch + b) * n + i];
-      y2[i] = L.y2[((long long)s * batch + b) * n + i];
+    if ((int)threadIdx.x < n) {
+      ref[threadIdx.x] = ref_next;
+      y1[threadIdx.x] = y1_next;
+      y2[threadIdx.x] = y2_next;
     }
     __syncthreads();
+    if (s + 1 < sec.n_sector) fetch(s + 1);
     // element (r, c) of the work matrix: the real part of logical (i, j), or in a complex call the part that its
     // place in the 2x2 block [[X, Z], [Z, -X]] asks for
-    const auto start = [&](int r, int c, double before) {  // phases 0 and 1: `before` is Y, or y2 S y2 of the last sector
+    const double h3 = h / 3.0, hp3 = hp / 3.0;
+    const auto imaginary = [&](int r, int c) { return cplx && ((r ^ c) & 1); };
+    const auto start_w = [&](int r, int c) {  // the part of phases 0 and 1 that comes from W
       const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
-      const bool imag = cplx && ((r ^ c) & 1);
-      const double d = (i == j) ? 1.0 : 0.0;
-      double x = before;
-      if (!imag) {
-        if (s > 0) x += hp * (Wep[(long long)i * n + j] - d * refp[i]) / 3.0 + d * y1p[i];
-        x += h * (Ws[(long long)i * n + j] - d * ref[i]) / 3.0 + d * y1[i];
-      }
+      if (imaginary(r, c)) return 0.0;
+      double x = h3 * (Ws[(long long)i * n + j] - (i == j ? ref[i] : 0.0));
+      if (s > 0) x += hp3 * (Wep[(long long)i * n + j] - (i == j ? refp[i] : 0.0));
+      return x;
+    };
+    const auto start = [&](int r, int c, double before, double w) {  // `before` is Y, or y2 S y2 of the last sector
+      const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+      const bool imag = imaginary(r, c);
+      double x = before + w;
+      if (!imag && i == j) x += s > 0 ? y1[i] + y1p[i] : y1[i];
       small_put<D>(S, r, c, (cplx && !imag && (r & 1)) ? -x : x);
     };
     // y2_i S_ij y2_j from the swept element of the same place (in a complex call -S on the imaginary places and on the
@@ -550,36 +573,43 @@ __global__ void __launch_bounds__(SmallShape<D>::kThreads, SmallShape<D>::kPerSM
         } else {
           v = 0.5 * (Yb[(long long)r * n + c] + Yb[(long long)c * n + r]);
         }
-        start(r, c, v);
+        start(r, c, v, start_w(r, c));
       }
       __syncthreads();
     } else {
-      singular |= small_sweep_then<D>(S, aux, used, [&](int r, int c, double v) { start(r, c, folded(r, c, v, y2p)); });
+      singular |= small_sweep_then<D>(S, aux, used, start_w, [&](int r, int c, double v, double w) { start(r, c, folded(r, c, v, y2p), w); });
     }
-    singular |= small_sweep_then<D>(S, aux, used, [&](int r, int c, double v) {
-      const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
-      const bool imag = cplx && ((r ^ c) & 1);
-      double x = folded(r, c, v, y2);
-      if (!imag) x += 2.0 * Q[(long long)i * L.npr + j] + (i == j ? 2.0 * y1[i] : 0.0);
-      small_put<D>(S, r, c, (cplx && !imag && (r & 1)) ? -x : x);
-    });
+    singular |= small_sweep_then<D>(
+        S, aux, used, [&](int r, int c) { return imaginary(r, c) ? 0.0 : 2.0 * Q[(long long)(cplx ? r >> 1 : r) * L.npr + (cplx ? c >> 1 : c)]; },
+        [&](int r, int c, double v, double w) {
+          const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+          const bool imag = imaginary(r, c);
+          double x = folded(r, c, v, y2) + w;
+          if (!imag && i == j) x += 2.0 * y1[i];
+          small_put<D>(S, r, c, (cplx && !imag && (r & 1)) ? -x : x);
+        });
     if (s + 1 == sec.n_sector) {
-      singular |= small_sweep_then<D>(S, aux, used, [&](int r, int c, double v) {
-        const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
-        const bool imag = cplx && ((r ^ c) & 1);
-        if (cplx && (r & 1) && !(imag && i == j)) return;  // the first row of each 2x2 block holds both parts (on the diagonal its
-                                                           // imaginary part is visited in the second)
-        const double d = (i == j) ? 1.0 : 0.0;
-        double x = folded(r, c, v, y2);
-        if (!imag) x += h * (We[(long long)i * n + j] - d * ref[i]) / 3.0 + d * y1[i];
-        if (cplx) {
-          Yb[2 * ((long long)i * n + j) + (imag ? 1 : 0)] = x;
-          Yb[2 * ((long long)j * n + i) + (imag ? 1 : 0)] = x;
-        } else {
-          Yb[(long long)i * n + j] = x;
-          Yb[(long long)j * n + i] = x;
-        }
-      });
+      singular |= small_sweep_then<D>(
+          S, aux, used,
+          [&](int r, int c) {
+            const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+            return imaginary(r, c) ? 0.0 : h3 * (We[(long long)i * n + j] - (i == j ? ref[i] : 0.0));
+          },
+          [&](int r, int c, double v, double w) {
+            const int i = cplx ? r >> 1 : r, j = cplx ? c >> 1 : c;
+            const bool imag = imaginary(r, c);
+            // the first row of each 2x2 block holds both parts (on the diagonal its imaginary part is visited in the second)
+            if (cplx && (r & 1) && !(imag && i == j)) return;
+            double x = folded(r, c, v, y2) + w;
+            if (!imag && i == j) x += y1[i];
+            if (cplx) {
+              Yb[2 * ((long long)i * n + j) + (imag ? 1 : 0)] = x;
+              Yb[2 * ((long long)j * n + i) + (imag ? 1 : 0)] = x;
+            } else {
+              Yb[(long long)i * n + j] = x;
+              Yb[(long long)j * n + i] = x;
+            }
+          });
     }
   }
   if (singular && threadIdx.x == 0) report_status(status, kDeviceSingularPivot, b, 0);
