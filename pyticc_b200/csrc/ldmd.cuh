@@ -217,6 +217,10 @@ __global__ void __launch_bounds__(kElemThreads) ldmd_elementwise_kernel(int s, i
   const int n = L.n, np = L.np, ne = L.n_energy, batch = L.n_block * ne;
   const int i0 = ta * kCols + (blockIdx.x % kGroups) * kElemRows, j0 = tb * kCols;
   const int e0 = blockIdx.y * e_per, e1 = min(ne, e0 + e_per);
+  // The W matrices, y1, y2 and (but for the first sector) Q_mid were complete before the sweep ahead of this pass began:
+  // their part is read while that sweep drains.
+  next_kernel_may_start();
+  if (s == 0) previous_kernel_done();
   if (kPhase == 3 && i0 >= n) return;
   const double h = sec.h[s];
   const long long wb = g * sec.wb_stride;
@@ -252,6 +256,7 @@ __global__ void __launch_bounds__(kElemThreads) ldmd_elementwise_kernel(int s, i
         base[r][q][c] = v;
       }
   }
+  previous_kernel_done();
   const int sy = kPhase == 1 ? s - 1 : s;  // the sector whose y1, y2 fold the swept matrix
   for (int e = e0; e < e1; e += 2) {
     const int cnt = min(2, e1 - e);
@@ -382,18 +387,14 @@ inline cudaError_t ldmd_elementwise(int phase, int s, const LdmdSectors& sec, co
   long long e_per = per_energy * L.n_energy / target;
   e_per = e_per < 1 ? 1 : e_per > L.n_energy ? L.n_energy : e_per;
   const dim3 grid((unsigned)tiles, (unsigned)((L.n_energy + e_per - 1) / e_per), (unsigned)L.n_block);
-#define TICC_ELEMENTWISE(P)                                                                                                                  \
-  if (L.is_complex) ldmd_elementwise_kernel<P, true><<<grid, kElemThreads, 0, stream>>>(s, (int)e_per, sec, L, Yin, Yout);  \
-  else ldmd_elementwise_kernel<P, false><<<grid, kElemThreads, 0, stream>>>(s, (int)e_per, sec, L, Yin, Yout);
-  switch (phase) {
-    case 0: TICC_ELEMENTWISE(0) break;
-    case 1: TICC_ELEMENTWISE(1) break;
-    case 2: TICC_ELEMENTWISE(2) break;
-    default: TICC_ELEMENTWISE(3) break;
-  }
-#undef TICC_ELEMENTWISE
+  const auto launch = [&](auto* real, auto* complex) { return launch_overlapped(L.is_complex ? complex : real, grid, kElemThreads, 0, stream, s, (int)e_per, sec, L, Yin, Yout); };
   note_launch();
-  return cudaGetLastError();
+  switch (phase) {
+    case 0: return launch(ldmd_elementwise_kernel<0, false>, ldmd_elementwise_kernel<0, true>);
+    case 1: return launch(ldmd_elementwise_kernel<1, false>, ldmd_elementwise_kernel<1, true>);
+    case 2: return launch(ldmd_elementwise_kernel<2, false>, ldmd_elementwise_kernel<2, true>);
+    default: return launch(ldmd_elementwise_kernel<3, false>, ldmd_elementwise_kernel<3, true>);
+  }
 }
 
 // ---- matrices of at most 128 rows: the whole call in one launch ----------------------------------------

@@ -1240,7 +1240,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) sweep_step_kernel(double* __r
   int* slot = reinterpret_cast<int*>(reinterpret_cast<char*>(smem) + kStepSlotOffset);
   int* queue = ints + (kb & 1);
   int* abort_flag = ints + 2;
-  if (blockIdx.x == 0 && tid == 0) ints[(kb + 1) & 1] = 0;  // the next step's queue
   const int per = t * (t + 1) / 2;
   const int n_panel = t * batch;
   const int n_pivot = fuse_next ? batch : 0;
@@ -1255,6 +1254,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) sweep_step_kernel(double* __r
     tc_setup(tcs, smem, ld);
     tc_live = true;
   }
+  previous_kernel_done();
+  if (blockIdx.x == 0 && tid == 0) ints[(kb + 1) & 1] = 0;  // the next step's queue
   for (;;) {
     // the previous unit's generic shared-memory writes come before any TMA load of the next
     if (tensor_core) fence_proxy_async_shared();
@@ -1417,7 +1418,8 @@ inline cudaError_t sweep_batched(double* M, long long mstride, int np, int batch
       const int fuse = (kb + 1 < nt) ? 1 : 0;
       const long long work = (long long)t * batch + (fuse ? batch : 0) + per * batch;
       const long long blocks = work < sms ? work : sms;
-      sweep_step_kernel<<<(unsigned)blocks, kGemmThreads, kStepSmemBytes, stream>>>(M, mstride, np, kb, cold, cstride, t, batch, fuse, pinv, status, reduced_blocks, queue, tc_split, maps);
+      e = launch_overlapped(sweep_step_kernel, (unsigned)blocks, kGemmThreads, kStepSmemBytes, stream, M, mstride, np, kb, cold, cstride, t, batch, fuse, pinv, status, reduced_blocks, queue, tc_split, maps);
+      if (e != cudaSuccess) return e;
       note_launch();
     }
     return cudaGetLastError();

@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
   const int per_step = batch * (t + t * (t + 1) / 2 - 1);  // the last step has `batch` more
   const int total = batch + per_step * nt + batch;
   const int tid = threadIdx.x;
+  previous_kernel_done();
   for (;;) {
     if (tid == 0) slot[0] = atomicAdd(w.control, 1) - w.queue_base;
     __syncthreads();
@@ -454,7 +455,8 @@ inline cudaError_t fine_sweep(FineState& state, double* M, long long mstride, in
   w.status = status;
   const long long total = (long long)batch + (long long)batch * (t + t * (t + 1) / 2 - 1) * nt + batch;
   // flag values and queue counts stay far below 2^31; another shape, or a long run of sweeps, starts afresh
-  if (state.sweeps == 0 || state.nt != nt || state.batch != batch || state.sweeps > 4096 || state.queue > (1 << 30)) {
+  const bool fresh = state.sweeps == 0 || state.nt != nt || state.batch != batch || state.sweeps > 4096 || state.queue > (1 << 30);
+  if (fresh) {
     e = cudaMemsetAsync(w.control, 0, kFineControlDoubles * sizeof(double), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.flags, 0, sizeof(int) * (size_t)batch * fine_flag_ints(nt), stream);
     if (e != cudaSuccess) return e;
@@ -472,11 +474,12 @@ inline cudaError_t fine_sweep(FineState& state, double* M, long long mstride, in
   const bool dense = (long long)batch * (t + t * (t + 1) / 2) > 4LL * sms;
   const long long slots = dense ? 2LL * sms : sms;
   const int grid = (int)(total < slots ? total : slots);
-  if (dense) sweep_fine_kernel<2><<<grid, kFineThreads, kFineSmemBytes, stream>>>(w);
-  else sweep_fine_kernel<1><<<grid, kFineThreads, kFineSmemBytes, stream>>>(w);
+  auto* kernel = dense ? sweep_fine_kernel<2> : sweep_fine_kernel<1>;
   note_launch();
   ++state.sweeps;
   state.queue += (int)total + grid;
+  if (!fresh) return launch_overlapped(kernel, grid, kFineThreads, kFineSmemBytes, stream, w);
+  kernel<<<grid, kFineThreads, kFineSmemBytes, stream>>>(w);  // behind the clearing of its flags
   return cudaGetLastError();
 }
 

@@ -44,6 +44,29 @@ inline std::atomic<long long>& launch_counter() {
 }
 inline void note_launch(long long n = 1) { launch_counter().fetch_add(n, std::memory_order_relaxed); }
 
+// Launch `kernel` so that its CTAs may come up while the kernel before it in the stream drains: the CTAs of a kernel launched so
+// call previous_kernel_done() before they touch anything that the call's earlier kernels write.  A kernel that starts
+// behind such a one and waits is ordered behind everything before it too, because the other finished only after its own wait.
+// Between the passes and sweeps of a propagation this hides the launch, the first loads and a sweep's thinning tail:
+// measured, N = 231, 16 energies, 8 sectors 1865 -> 1808 us, a rigid-rotor solve of 24 sectors 7.96 -> 7.69 ms, mixed windows of N = 1860 24.7 -> 24.5 ms.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = dim3((unsigned)threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+__device__ __forceinline__ void previous_kernel_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel's CTAs may come up as soon as every CTA of this one has said so.
+__device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 inline __host__ __device__ long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
 // Record the first device-side error: status[0] = code, status[1] = batch item,
