@@ -183,7 +183,8 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(const double* src,
 // then eliminates it while the others update theirs.
 // Pivot choice: the largest magnitude by its leading 24 bits (13 of mantissa) among the unused rows, the smallest row
 // on ties; a NaN or an infinity ranks above all and is reported, as is a zero (or subnormal) pivot.
-// gauss_jordan_exchange leaves S in exchange form: inverse element (j, m) is S[perm[j] * Ld + iperm[m]] (j, m < n_act).
+// gauss_jordan_exchange leaves S in exchange form: inverse element (j, m) is S[perm[j] * Ld + iperm[m]]
+// (rows and columns from n_act on, decoupled, as they were).
 struct GJOrder {
   const int* perm;
   const int* iperm;
@@ -200,6 +201,7 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
   bool singular = false;
   const int panels = n_act / kGJPanel;
   unsigned long long used = n_act == 64 ? 0ull : ~0ull << n_act;  // rows of all panels so far
+  if (t >= n_act && t < D) perm[t] = t;
   GJStrip<D> g;
   gj_load_strip<Ld, D>(g, S, kGJPanel * warp);
   __syncwarp();
@@ -239,7 +241,7 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
     }
     if (warp == q) {
       gj_load_strip<Ld, D>(g, S, j0);
-    } else if (warp < panels && warp != next) {
+    } else if (warp != next) {
       gj_update_strip<Ld, D>(g, S, perm + j0, kGJPanel * warp, j0, mask);
       if (warp == next + 1) {  // the panel after the next: to its place
         __syncwarp();
@@ -248,8 +250,8 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
     }
   }
   __syncthreads();  // the last panel's E has been read
-  if (warp < panels) gj_store_strip<Ld, D>(g, S, kGJPanel * warp);
-  if (t < n_act) iperm[perm[t]] = t;
+  gj_store_strip<Ld, D>(g, S, kGJPanel * warp);
+  if (t < D) iperm[perm[t]] = t;
   order.perm = perm;
   order.iperm = iperm;
   return __syncthreads_or(singular);
