@@ -300,17 +300,11 @@ int ticc_contract(const double* rows_real, const double* rows_imag, const int* g
   ticc::contract_init_kernel<<<ticc::grid_for((long long)n_R * n_channel * n_channel, 256), 256, 0, s>>>(out, n_channel, n_R, radial_points, U, E_int, reduced_mass);
   ticc::note_launch();
   const double scale = normalization * (U != nullptr ? 2.0 * reduced_mass : 1.0);
-  cudaError_t e = cudaFuncSetAttribute(ticc::contract_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ticc::kVSmemBytes);
-  if (e != cudaSuccess) return cuda_fail(e, "ticc_contract");
   // one launch per kVMaxGroups non-empty groups (and per 65535 radial points)
+  cudaError_t e = cudaSuccess;
   ticc::ContractTiles tiles{};
   auto flush = [&]() {
-    const int n_tiles = tiles.tile_start[tiles.n_groups];
-    for (int r0 = 0; r0 < n_R; r0 += 65535) {
-      ticc::contract_group_kernel<<<dim3(n_tiles, std::min(65535, n_R - r0)), ticc::kVThreads, ticc::kVSmemBytes, s>>>(tiles, rows_real, rows_imag, row_out, n_grid, scale, potential,
-                                                                                                                 pot_stride, r0, n_channel, out);
-      ticc::note_launch();
-    }
+    if (e == cudaSuccess) e = ticc::contract_groups(tiles, rows_real, rows_imag, row_out, n_grid, scale, potential, pot_stride, n_R, n_channel, out, s);
     tiles.n_groups = 0;
     tiles.tile_start[0] = 0;
   };
@@ -325,7 +319,7 @@ int ticc_contract(const double* rows_real, const double* rows_imag, const int* g
     if (tiles.n_groups == ticc::kVMaxGroups) flush();
   }
   if (tiles.n_groups > 0) flush();
-  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? TICC_OK : cuda_fail(e, "ticc_contract");
 }
 
@@ -338,11 +332,11 @@ int ticc_contract_block(const double* A, int n_a, const double* B, int n_b, int 
     return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_contract_block: n_a=%d n_b=%d n_grid=%d n_R=%d n=%d w_stride=%lld symmetric=%d (a symmetric block has B = A)", n_a, n_b,
                 n_grid, n_R, n, w_stride, symmetric);
   if (n_a == 0 || n_b == 0 || n_R == 0) return TICC_OK;
-  cudaError_t e = cudaFuncSetAttribute(ticc::weighted_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ticc::kVSmemBytes);
+  cudaError_t e = cudaFuncSetAttribute(ticc::weighted_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ticc::kVSmemBytes<1>);
   if (e != cudaSuccess) return cuda_fail(e, "ticc_contract_block");
   for (int r0 = 0; r0 < n_R; r0 += 65535) {
     const dim3 grid((n_a + ticc::kVTile - 1) / ticc::kVTile, (n_b + ticc::kVTile - 1) / ticc::kVTile, std::min(65535, n_R - r0));
-    ticc::weighted_block_kernel<<<grid, ticc::kVThreads, ticc::kVSmemBytes, as_stream(stream)>>>(A, n_a, B, n_b, n_grid, weights, w_stride, r0, pos_a, pos_b, symmetric, mirror, n, out);
+    ticc::weighted_block_kernel<<<grid, ticc::kVThreads, ticc::kVSmemBytes<1>, as_stream(stream)>>>(A, n_a, B, n_b, n_grid, weights, w_stride, r0, pos_a, pos_b, symmetric, mirror, n, out);
     ticc::note_launch();
   }
   e = cudaGetLastError();
