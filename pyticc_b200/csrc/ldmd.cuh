@@ -403,8 +403,8 @@ inline cudaError_t ldmd_elementwise(int phase, int s, const LdmdSectors& sec, co
 // one CTA keeps its (block, energy) matrix in shared memory through every sector of the call: the elementwise passes
 // run between inversions on the tile itself, and only W, Q_mid, y1 and y2 are read.  D = 32 or 64: Gauss-Jordan
 // exchange, whose permuted result the next pass reads in place; D = 128: the two-level sweep_block.
-// Measured (B200), propagate_logD of N = 21, 1 energy, 16 sectors: 898 -> 397 us a call; coupled-states blocks of 1 to 21
-// channels, 16 energies, 12 sectors: 5.7 -> 4.1 ms a call (the rest is the host's per-block work).
+// Measured (B200), propagate_logD of N = 21, 1 energy, 16 sectors: 898 -> 363 us a call; coupled-states blocks of 1 to 21
+// channels, 16 energies, 12 sectors: 5.7 -> 4.1 ms a call (the rest was the host's per-block work: 1.7 ms since that is shared).
 template <int D>
 struct SmallShape {
   static constexpr int kThreads = D == 32 ? 128 : 256;
