@@ -196,6 +196,14 @@ __device__ __forceinline__ void fine_sub(FineAcc& c, const FineAcc& d) {
       c.v[u][w][1] -= d.v[u][w][1];
     }
 }
+// By one thread behind a __syncthreads(): count a finished update of this step.  The fence orders the reads of its panel tiles (the
+// whole CTA's, through the barrier) before the count, on which the chain waits before it has the slots written again; with
+// `version` it publishes the updated tile too, so that the two cost one fence.
+__device__ __forceinline__ void fine_count_update(int* done, int* version = nullptr, int value = 0) {
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  if (version != nullptr) asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(version), "r"(value) : "memory");
+  asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(done) : "memory");
+}
 // Call f(row, column, double2 of the accumulator) for every pair this lane holds.
 template <class F>
 __device__ __forceinline__ void fine_each(FineAcc& acc, F&& f) {
@@ -368,7 +376,7 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       // M(j, j) - X R^T (here j = k + 1 > k: X[c][k], R[c][k]), lower half, mirrored
       fine_lower_update(SA, SC, SA, Mb + (long long)j * kSub * w.ld + j * kSub, w.ld);
       __syncthreads();
-      if (tid == kFineThreads - 64) atomicAdd(done + k, 1);
+      if (tid == kFineThreads - 64) fine_count_update(done + k);
       fine_invert(w, b, j, SA, SC, aux, Mb, f + 2 * nt, const_cast<int*>(ver) + fine_lower(j, j), now + 2);
       continue;
     }
@@ -417,10 +425,7 @@ __global__ void __launch_bounds__(kFineThreads, kPerSM) sweep_fine_kernel(const 
       }
     });
     __syncthreads();
-    if (tid == 0) {
-      store_release(const_cast<int*>(ver) + fine_lower(ta, tb), now + 1);
-      atomicAdd(done + k, 1);
-    }
+    if (tid == 0) fine_count_update(done + k, const_cast<int*>(ver) + fine_lower(ta, tb), now + 1);
   }
 }
 
