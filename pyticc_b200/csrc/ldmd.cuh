@@ -187,6 +187,12 @@ __device__ __forceinline__ void get_swept(const double* Mb, int np, int i, int j
 // Work-matrix padding: identity on the padded diagonal of the real sweep matrix.
 __device__ __forceinline__ void put_padding(double* Mb, int np, long long r, long long c) { Mb[r * np + c] = (r == c) ? 1.0 : 0.0; }
 
+// One complex element of the caller's Y, which need not be 16-byte aligned.
+__device__ __forceinline__ void put_pair(double* y, double re, double im) {
+  y[0] = re;
+  y[1] = im;
+}
+
 // W_base must be exactly symmetric (the contraction writes both halves from one value), so the per-energy passes read
 // W[i][j] only, row-contiguous across the lanes of a warp.
 // phase 0: A = Y_in + Q_start + y1          (first sector of the call)
@@ -352,7 +358,7 @@ __global__ void __launch_bounds__(kElemThreads) ldmd_elementwise_kernel(int s, i
             double* Yo = Yout + (long long)b * n * n * (kCplx ? 2 : 1);
             const long long at = (long long)i[r] * n + j;
             if (kCplx) {
-              if (row_in && j < n) *reinterpret_cast<double2*>(Yo + 2 * at) = x;
+              if (row_in && j < n) put_pair(Yo + 2 * at, x.x, x.y);
               strip[jj * (kElemRows + 1) + ii] = x.x;
               strip[(kCols + jj) * (kElemRows + 1) + ii] = x.y;
             } else {
@@ -371,7 +377,7 @@ __global__ void __launch_bounds__(kElemThreads) ldmd_elementwise_kernel(int s, i
           const int jj = t / kElemRows, ii = t % kElemRows;
           if (j0 + jj >= n || i0 + ii >= n) continue;
           const long long at = (long long)(j0 + jj) * n + i0 + ii;
-          if (kCplx) *reinterpret_cast<double2*>(Yo + 2 * at) = make_double2(strip[jj * (kElemRows + 1) + ii], strip[(kCols + jj) * (kElemRows + 1) + ii]);
+          if (kCplx) put_pair(Yo + 2 * at, strip[jj * (kElemRows + 1) + ii], strip[(kCols + jj) * (kElemRows + 1) + ii]);
           else Yo[at] = strip[jj * (kElemRows + 1) + ii];
         }
       }
