@@ -98,13 +98,14 @@ def blocks_workspace_bytes(n: int, n_energy: int, n_block: int, n_sector: int, i
     return nat.size_query(nat.load_library().ticc_ldmd_blocks_workspace_size, n, n_energy, n_block, n_sector, int(is_complex), precision)
 
 
-def propagate_blocks_device(Y: torch.Tensor, energies: torch.Tensor, reduced_mass: float, half_steps: torch.Tensor, W_start: torch.Tensor, W_mid: torch.Tensor, W_end: torch.Tensor, *, stride, block_stride: int, precision: int = nat.PRECISION_FP64, workspace_slot: int = 0, status: "nat.DeviceStatus | None" = None) -> torch.Tensor:
+def propagate_blocks_device(Y: torch.Tensor, energies: torch.Tensor, reduced_mass: float, half_steps: torch.Tensor, W_start: torch.Tensor, W_mid: torch.Tensor, W_end: torch.Tensor, *, stride, block_stride: int, precision: int = nat.PRECISION_FP64, workspace_slot: int = 0, workspace: torch.Tensor | None = None, status: "nat.DeviceStatus | None" = None) -> torch.Tensor:
     """Propagate device-resident Y of shape (n_block, n_energy, n, n) in place: block g
     reads its W at element offset g * block_stride from the three W views, whose
     consecutive sectors are ``stride`` elements apart.  Calls that may run concurrently on
-    different streams pass different ``workspace_slot``s.  With ``status`` (a DeviceStatus
-    the caller checks later) the call neither allocates a status word nor synchronises, so
-    it can be captured into a CUDA graph once its workspace slot is large enough."""
+    different streams pass different ``workspace_slot``s, or a ``workspace`` (uint8, of
+    ``blocks_workspace_bytes``) of their own.  With ``status`` (a DeviceStatus the caller checks
+    later) the call neither allocates a status word nor synchronises: with a workspace that
+    lives as long as the graph, it can be captured into a CUDA graph."""
     lib = nat.load_library()
     n_block, n_energy, n, _ = Y.shape
     n_sector = half_steps.numel()
@@ -112,8 +113,10 @@ def propagate_blocks_device(Y: torch.Tensor, energies: torch.Tensor, reduced_mas
     dev = Y.device
     check_now = status is None
     with torch.cuda.device(dev):
-        nbytes = blocks_workspace_bytes(n, n_energy, n_block, n_sector, bool(is_complex), precision)
-        work = nat.Workspace.get(dev, nbytes, slot=workspace_slot)
+        work = workspace
+        if work is None:
+            nbytes = blocks_workspace_bytes(n, n_energy, n_block, n_sector, bool(is_complex), precision)
+            work = nat.Workspace.get(dev, nbytes, slot=workspace_slot)
         status = nat.DeviceStatus(dev) if status is None else status
         nat.check(
             lib.ticc_ldmd_propagate_blocks(

@@ -38,7 +38,6 @@ from .grid import MAX_SECTORS_PER_WINDOW, RadialSector, radial_points_of
 from .logd import blocks_workspace_bytes, propagate_blocks_device
 from .runner import BlockState, DeviceBlocks, initial_logD
 
-SWEEP_WORKSPACE_SLOT = 32     # workspace slot shared by the sweep's launches (they run in order)
 PROBE_SECTORS = 2             # sectors timed per option by the autotuner
 _AUTOTUNE: dict = {}          # (device name, mode, precision, n_energy, class signature) -> merge decisions
 
@@ -123,9 +122,10 @@ class _Launch:
         self.Y = torch.empty((self.n_block, n_energy, n, n), dtype=dtype, device=device)
         self.energies = torch.zeros(n_energy, dtype=torch.float64, device=device)
         self.status = nat.DeviceStatus(device)
-        self.workspace_bytes = blocks_workspace_bytes(n, n_energy, self.n_block, size, self.complex, self.precision)
+        counts = {count for count, *_ in self.windows}
+        self.workspace_bytes = max(blocks_workspace_bytes(n, n_energy, self.n_block, count, self.complex, self.precision) for count in counts)
 
-    def enqueue(self) -> None:
+    def enqueue(self, workspace: torch.Tensor) -> None:
         db = self.db
         stride = 2 * self.n * self.n
         for w, (count, index, R, halves) in enumerate(self.windows):
@@ -137,7 +137,7 @@ class _Launch:
                 for g in range(self.n_block):
                     self.Y[g].copy_(initial_logD(self.W[g, 0], self.energies, db.reduced_mass, self.config.mode))
             propagate_blocks_device(self.Y, self.energies, db.reduced_mass, halves, self.W[0, 0], self.W[0, 1], self.W[0, 2], stride=(stride, stride, stride),
-                                    block_stride=self.points_max * self.n * self.n, precision=self.precision, workspace_slot=SWEEP_WORKSPACE_SLOT, status=self.status)
+                                    block_stride=self.points_max * self.n * self.n, precision=self.precision, workspace=workspace, status=self.status)
 
     def block_Y(self, g: int) -> torch.Tensor:
         size = self.db.sizes[g]
@@ -223,7 +223,8 @@ class PartialWaveSweep:
         self.merges = merges
         self.launches = [_Launch([self.states[i] for i in p.members], p.n, self.sectors, self.n_energy, self.energy_bound, propagation, self.device) for p in plans]
         self.members = [p.members for p in plans]
-        nat.Workspace.get(self.device, max(l.workspace_bytes for l in self.launches), slot=SWEEP_WORKSPACE_SLOT)
+        # one workspace for the launches (they run in order), held here: the graph replays into its address
+        self.workspace = torch.empty(max(l.workspace_bytes for l in self.launches), dtype=torch.uint8, device=self.device)
         self.use_graph = graph
         self.graph = None
         self.graph_launches = 0  # library kernels recorded in the graph (each replay launches them)
@@ -241,12 +242,12 @@ class PartialWaveSweep:
     def _probe(self, members: Sequence[int], n: int) -> float:
         """Device milliseconds of PROBE_SECTORS sectors of one launch of these blocks."""
         launch = _Launch([self.states[i] for i in members], n, self.sectors[:PROBE_SECTORS], self.n_energy, self.energy_bound, self.config, self.device)
-        nat.Workspace.get(self.device, launch.workspace_bytes, slot=SWEEP_WORKSPACE_SLOT)
+        workspace = torch.empty(launch.workspace_bytes, dtype=torch.uint8, device=self.device)
         launch.energies.fill_(0.5 * self.energy_bound)
-        launch.enqueue()  # warm
+        launch.enqueue(workspace)  # warm
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
-        launch.enqueue()
+        launch.enqueue(workspace)
         stop.record()
         torch.cuda.synchronize(self.device)
         launch.status.raise_if_failed("partial-wave sweep autotune probe")
@@ -285,7 +286,7 @@ class PartialWaveSweep:
     # ---- running -----------------------------------------------------------------------------
     def _enqueue_all(self) -> None:
         for launch in self.launches:
-            launch.enqueue()
+            launch.enqueue(self.workspace)
 
     def propagate(self, Etot) -> list[torch.Tensor | None]:
         """Y at the last sector end for every block (device, original channel order)."""
