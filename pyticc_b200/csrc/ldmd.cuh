@@ -415,7 +415,7 @@ template <int D>
 struct SmallShape {
   static constexpr int kThreads = D == 32 ? 128 : 256;
   static constexpr int kLd = D + 4;
-  static constexpr size_t kAux = D == 128 ? kPivotAuxBytes / sizeof(double) : kGJAuxDoubles;
+  static constexpr size_t kAux = D == 128 ? kPivotAuxBytes / sizeof(double) : kGJAuxDoubles + size_t(D) * kLd;
   static constexpr size_t kSmemBytes = (size_t(D) * kLd + kAux + 6 * D) * sizeof(double);
   static constexpr int kPer = D == 128 ? 1 : D * D / kThreads;
   static constexpr int kPerSM = D == 32 ? 4 : D == 64 ? 2 : 1;
@@ -446,7 +446,7 @@ __device__ inline bool small_sweep_then(double* S, double* aux, int used, P&& pr
       w[u] = (D == 32 && r < used && c <= r) ? pre(r, c) : 0.0;  // (64 rows: the registers are the exchange's)
     }
     GJOrder order;
-    const bool singular = gauss_jordan_exchange<Sh::kLd, Sh::kThreads, D>(S, aux, order, n_act);
+    const bool singular = gauss_jordan_exchange<Sh::kLd, Sh::kThreads, D>(S, aux, aux + kGJAuxDoubles, order, n_act);
 #pragma unroll
     for (int u = 0; u < Sh::kPer; ++u) {
       const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;

@@ -89,9 +89,11 @@ __device__ __forceinline__ void gj_update_strip(GJStrip<D>& g, double* S, const 
   }
 }
 
-// 1/a for a normal a (subnormal results flush to zero): the hardware's approximation y (relative error 2^-23) and one step of the
-// third-order Newton (Householder) iteration y (1 + e + e^2), e = 1 - a y, whose own error is e^3.  Four instructions
-// and no branch, so that the search around it can be scheduled into its latency (the divide operator ends a basic block).
+// 1/a where a and 1/a are normal numbers (nothing in it handles others): the hardware's approximation y, which reads and
+// writes the upper 32 bits only (relative error about 2^-20), and one step of the third-order Newton (Householder) iteration
+// y (1 + e + e^2), e = 1 - a y, whose own error is e^3, about 2^-60: with the last rounding 1/a to within a unit in the last
+// place.  Four instructions and no branch, so that the search around it can be scheduled into its latency (the divide
+// operator ends a basic block).
 __device__ __forceinline__ double gj_reciprocal(double a) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
@@ -99,14 +101,17 @@ __device__ __forceinline__ double gj_reciprocal(double a) {
   return fma(y, fma(e, e, e), y);
 }
 
+// Ranks (exponent field first) of the pivots that it takes: 2^-1022 <= |a| < 2^1021.
+constexpr unsigned kGJFirst = 1u << 21, kGJSpan = (0x7fcu << 21) - kGJFirst;
+
 // Eliminate the panel that becomes columns j0 .. j0 + 7 of S by one warp (exchange steps inside the panel only); src: the
 // panel's values (row stride src_ld).  Lane l holds
 // rows l and, where D = 64, l + 32; rows in `rows_before` have been pivots (or do not take part).  Returns the panel's pivot rows as
-// a mask; prow[0..7] gets them in order.
+// a mask; prow[0..7] gets them in order; `outside` is set (and the panel garbage) where a pivot was beyond gj_reciprocal's range.
 template <int Ld, int D>
-__device__ __forceinline__ unsigned long long gj_factor_panel(const double* src, int src_ld, double* S, int* prow, int j0, unsigned long long rows_before, bool& singular) {
+__device__ __forceinline__ unsigned long long gj_factor_panel(const double* src, int src_ld, double* S, int* prow, int j0, unsigned long long rows_before, bool& outside) {
   const int lane = threadIdx.x & 31;
-  // rank of a row: its magnitude's leading 24 bits, then its index (the smaller row wins); 0 for a used row
+  // rank of a row: its magnitude's leading 25 bits (14 of mantissa), then its index (the smaller row wins); 0 for a used row
   constexpr unsigned kRankMask = ~127u;
   unsigned mask0 = ((rows_before >> lane) & 1ull) ? 0u : kRankMask, mask1 = D == 32 || ((rows_before >> (lane + 32)) & 1ull) ? 0u : kRankMask;
   unsigned code0 = mask0 ? 127u - lane : 0u, code1 = mask1 ? 95u - lane : 0u;
@@ -127,8 +132,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(const double* src,
     const bool second = D == 64 && h1 > h0;
     const unsigned key = second ? h1 : h0;
     const unsigned best = __reduce_max_sync(0xffffffffu, key);
-    constexpr unsigned kFirst = 1u << 21, kSpan = 0xffe00000u - kFirst;  // ranks of normal finite magnitudes
-    const double inv_own = gj_reciprocal((key - kFirst) < kSpan ? (second ? v1[0] : v0[0]) : 1.0);  // of every lane's candidate, beside the search
+    const double inv_own = gj_reciprocal((key - kGJFirst) < kGJSpan ? (second ? v1[0] : v0[0]) : 1.0);  // of every lane's candidate, beside the search
     const int row = 127 - (int)(best & 127u);
     const bool upper = D == 64 && row >= 32;  // the half that holds the pivot row: the same for all lanes
     double p[kGJPanel];
@@ -140,7 +144,7 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(const double* src,
     code0 = own0 ? 0u : code0;
     mask1 = own1 ? 0u : mask1;
     code1 = own1 ? 0u : code1;
-    singular |= !((best - kFirst) < kSpan);
+    outside |= !((best - kGJFirst) < kGJSpan);
     if (lane == 0) prow[jj] = row;
     // the pivot row starts from zero with f = 1/a, every other row takes f = v/a
 #pragma unroll
@@ -169,9 +173,76 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(const double* src,
   return all & ~rows_before;
 }
 
+// Copy of a strip in the order of its registers (D x D doubles in all): conflict-free (at row stride D + 4 the copy cost 1 % of a sweep).
+template <int D>
+__device__ __forceinline__ void gj_save_strip(const GJStrip<D>& g, double* save) {
+#pragma unroll
+  for (int mt = 0; mt < D / 8; ++mt) reinterpret_cast<double2*>(save)[((threadIdx.x >> 5) * (D / 8) + mt) * 32 + (threadIdx.x & 31)] = g.v[mt];
+}
+template <int D>
+__device__ __forceinline__ double gj_saved(const double* save, int r, int c) {
+  return save[2 * (((c >> 3) * (D / 8) + (r >> 3)) * 32 + (r & 7) * 4 + ((c & 7) >> 1)) + (c & 1)];
+}
+
+// The exchange below, column by column, from the copy of the block in `save`: for blocks with a pivot that is
+// subnormal, 2^1021 or more, or not finite.  Pivot: the largest magnitude (a NaN above all), the smallest row on ties; its
+// reciprocal is formed at a scale where both are normal.  Returns true if a pivot was zero or non-finite.
+// Inlined behind the fast exchange's last barrier and without a divide operator: a call anywhere in the kernel, or a branch to
+// the careful way inside a panel, slowed the fast exchange (N = 1000: 382 -> 406 us a sweep; as it stands 384, the
+// copy of the block being most of it).
+template <int Ld, int kThreads, int D>
+__device__ __forceinline__ bool gauss_jordan_any_range(double* S, const double* save, int* perm, int n_act) {
+  constexpr int kPer = D * D / kThreads;
+  const int t = threadIdx.x, lane = t & 31;
+  bool singular = false;
+  unsigned long long used = n_act == 64 ? 0ull : ~0ull << n_act;
+#pragma unroll 1
+  for (int u = 0; u < kPer; ++u) {
+    const int e = t + u * kThreads, r = e / D, c = e % D;
+    S[r * Ld + c] = gj_saved<D>(save, r, c);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int j = 0; j < n_act; ++j) {
+    // every warp finds the pivot for itself; rank: 1 + the magnitude's bits, 0 for a used row
+    const int row1 = (lane + 32) & (D - 1);
+    const unsigned long long r0 = (used >> lane) & 1ull ? 0ull : 1ull + (unsigned long long)__double_as_longlong(fabs(S[lane * Ld + j]));
+    const unsigned long long r1 = D == 32 || ((used >> row1) & 1ull) ? 0ull : 1ull + (unsigned long long)__double_as_longlong(fabs(S[row1 * Ld + j]));
+    const unsigned long long key = r1 > r0 ? r1 : r0;
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key, own = r1 > r0 ? row1 : lane;
+    const unsigned hmax = __reduce_max_sync(0xffffffffu, hi), lmax = __reduce_max_sync(0xffffffffu, hi == hmax ? lo : 0u);
+    const int p = (int)__reduce_min_sync(0xffffffffu, hi == hmax && lo == lmax ? own : 0xffffffffu);
+    used |= 1ull << p;
+    double a = S[p * Ld + j];
+    if (!(fabs(a) > 0.0) || !isfinite(a)) {
+      singular = true;
+      a = 1.0;
+    }
+    const double scale = fabs(a) < 0x1p-1022 ? 0x1p64 : fabs(a) < 0x1p1021 ? 1.0 : 0x1p-64;
+    const double inv = gj_reciprocal(a * scale) * scale;
+    double x[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int e = t + u * kThreads, r = e / D, c = e % D;
+      const double f = (r == p ? 1.0 : S[r * Ld + j]) * inv;
+      x[u] = c == j ? f : fma(-f, S[p * Ld + c], r == p ? 0.0 : S[r * Ld + c]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int e = t + u * kThreads, r = e / D, c = e % D;
+      if (r < n_act && c < n_act) S[r * Ld + c] = x[u];
+    }
+    if (t == 0) perm[j] = p;
+    __syncthreads();
+  }
+  return singular;
+}
+
 // S <- S^{-1} (D x D in shared memory, D = 32 or 64, row stride Ld = 4 mod 16) by Gauss-Jordan exchange with partial pivoting over
 // the block's rows, by the kThreads threads of the CTA.  `n_act` (a multiple of kGJPanel): rows and columns at or beyond
-// it hold the identity and are left alone.  Returns true if a pivot was zero or non-finite.  Uses named barrier 1.
+// it hold the identity and are left alone.  `save` (D x D): scratch, receives a copy of the block beside the first
+// panel's elimination.  Returns true if a pivot was zero or non-finite.  Uses named barrier 1.
 //
 // The exchange of one column is a serial chain (rank the rows, reciprocal, publish the row, update), so the work around
 // that chain is what costs.  It is blocked: one warp eliminates a panel of 8 columns in registers, with no barrier, no
@@ -181,8 +252,8 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(const double* src,
 // that a panel costs one CTA barrier.  The strip that is the next panel is updated by four warps together (one on each
 // SM sub-partition, 4 tile products instead of 16 in the chain), from its place in S into a buffer; its owner
 // then eliminates it while the others update theirs.
-// Pivot choice: the largest magnitude by its leading 24 bits (13 of mantissa) among the unused rows, the smallest row
-// on ties; a NaN or an infinity ranks above all and is reported, as is a zero (or subnormal) pivot.
+// Pivot choice: the largest magnitude by its leading 25 bits (14 of mantissa) among the unused rows, the smallest row
+// on ties; a NaN or an infinity ranks above all and is reported, as is a zero pivot.
 // gauss_jordan_exchange leaves S in exchange form: inverse element (j, m) is S[perm[j] * Ld + iperm[m]]
 // (rows and columns from n_act on, decoupled, as they were).
 struct GJOrder {
@@ -190,7 +261,7 @@ struct GJOrder {
   const int* iperm;
 };
 template <int Ld, int kThreads, int D = kSub>
-__device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& order, int n_act = D) {
+__device__ inline bool gauss_jordan_exchange(double* S, double* aux, double* save, GJOrder& order, int n_act = D) {
   static_assert(kThreads / 32 == D / kGJPanel, "a strip for every warp");
   constexpr int kWarps = kThreads / 32, kTiles = D / 8 / 4;  // row tiles of the next panel that each of its four warps updates
   unsigned long long* panel_rows = reinterpret_cast<unsigned long long*>(aux);  // [kSub / kGJPanel]
@@ -198,15 +269,16 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
   int* iperm = perm + kSub;
   double* panel = aux + kSub / kGJPanel + kSub;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, mr = lane >> 2, kr = lane & 3;
-  bool singular = false;
+  bool outside = false;
   const int panels = n_act / kGJPanel;
   unsigned long long used = n_act == 64 ? 0ull : ~0ull << n_act;  // rows of all panels so far
   if (t >= n_act && t < D) perm[t] = t;
   GJStrip<D> g;
   gj_load_strip<Ld, D>(g, S, kGJPanel * warp);
+  gj_save_strip<D>(g, save);
   __syncwarp();
   if (warp == 0) {
-    const unsigned long long m = gj_factor_panel<Ld, D>(S, Ld, S, perm, 0, used, singular);
+    const unsigned long long m = gj_factor_panel<Ld, D>(S, Ld, S, perm, 0, used, outside);
     if (lane == 0) panel_rows[0] = m;
   }
 #pragma unroll 1
@@ -232,7 +304,7 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
         }
         if (part == 0) {
           asm volatile("bar.sync 1, 128;" ::: "memory");
-          const unsigned long long m = gj_factor_panel<Ld, D>(panel, kGJNextLd, S, perm + kGJPanel * next, kGJPanel * next, used, singular);
+          const unsigned long long m = gj_factor_panel<Ld, D>(panel, kGJNextLd, S, perm + kGJPanel * next, kGJPanel * next, used, outside);
           if (lane == 0) panel_rows[next] = m;
         } else {
           asm volatile("bar.arrive 1, 128;" ::: "memory");
@@ -254,12 +326,18 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& or
   if (t < D) iperm[perm[t]] = t;
   order.perm = perm;
   order.iperm = iperm;
-  return __syncthreads_or(singular);
+  bool singular = false;
+  if (__syncthreads_or(outside)) {
+    singular = gauss_jordan_any_range<Ld, kThreads, D>(S, save, perm, n_act);
+    if (t < D) iperm[perm[t]] = t;
+    __syncthreads();
+  }
+  return singular;
 }
 template <int Ld, int kThreads>
-__device__ inline bool gauss_jordan_sub(double* S, double* aux, int n_act = kSub) {
+__device__ inline bool gauss_jordan_sub(double* S, double* aux, double* save, int n_act = kSub) {
   GJOrder order;
-  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, order, n_act);
+  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, save, order, n_act);
   constexpr int kPer = kSub * kSub / kThreads;
   double x[kPer];
 #pragma unroll
@@ -325,7 +403,7 @@ __device__ inline bool sweep_block(double* P, double* aux, int n_act = kBlock) {
     double* Pkr = P + k0 * kPivotLd + r0;
     double* Prk = P + r0 * kPivotLd + k0;
     double* Prr = P + r0 * kPivotLd + r0;
-    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj, s == 0 ? kSub : n_act - kSub);
+    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj, U, s == 0 ? kSub : n_act - kSub);
     small_gemm64(U, kSmallLd, Pkk, kPivotLd, Pkr, kPivotLd, 1.0, false);     // U = P_KK^-1 P_KR
     small_gemm64(Prr, kPivotLd, Prk, kPivotLd, U, kSmallLd, -1.0, true);  // P_RR -= P_RK U
     if (!kSym) small_gemm64(Prk, kPivotLd, Prk, kPivotLd, Pkk, kPivotLd, 1.0, false);  // V = P_RK P_KK^-1
@@ -400,13 +478,13 @@ __global__ void __launch_bounds__(kPivotThreads) sweep_pivot_kernel(double* __re
 
 // Sweep of a single-block matrix whose channels fill at most the leading 64 rows and
 // columns (the rest is identity padding): only the 64x64 block is inverted, in a CTA with
-// 36 KB of shared memory so that several matrices share an SM; the padding becomes -I.
-constexpr size_t kPivot64SmemBytes = (size_t(kSub) * kSmallLd + kGJAuxDoubles) * sizeof(double);
+// 75 KB of shared memory so that two matrices share an SM (its registers hold no third); the padding becomes -I.
+constexpr size_t kPivot64SmemBytes = (size_t(2) * kSub * kSmallLd + kGJAuxDoubles) * sizeof(double);
 template <bool kSym>
 __global__ void __launch_bounds__(kPivotThreads) sweep_pivot64_kernel(double* __restrict__ M, long long mstride, int ld, int n_act, int* status) {
   extern __shared__ double smem[];
   double* S = smem;
-  double* gj = S + kSub * kSmallLd;
+  double* gj = S + 2 * kSub * kSmallLd;
   const int b = blockIdx.x;
   double* Mb = M + (long long)b * mstride;
 #pragma unroll
@@ -415,7 +493,7 @@ __global__ void __launch_bounds__(kPivotThreads) sweep_pivot64_kernel(double* __
     *reinterpret_cast<double2*>(S + (piece >> 5) * kSmallLd + (piece & 31) * 2) = *reinterpret_cast<const double2*>(Mb + (long long)(piece >> 5) * ld + (piece & 31) * 2);
   }
   __syncthreads();
-  const bool singular = gauss_jordan_sub<kSmallLd, kPivotThreads>(S, gj, n_act);
+  const bool singular = gauss_jordan_sub<kSmallLd, kPivotThreads>(S, gj, S + kSub * kSmallLd, n_act);
   if (singular && threadIdx.x == 0) report_status(status, kDeviceSingularPivot, b, 0);
   for (int idx = threadIdx.x; idx < ld * ld; idx += kPivotThreads) {
     const int i = idx / ld, j = idx % ld;

@@ -219,11 +219,11 @@ __device__ __forceinline__ void fine_each(FineAcc& acc, F&& f) {
 __device__ __forceinline__ bool fine_mirrors(int ta, int tb, bool last) { return last && ta == tb + 1 && (tb & 1) == 0; }
 
 // Invert the symmetric block in S; publish P^{-1} first (`pivot_flag`, on which the chain waits), then write -P^{-1} into
-// M's diagonal tile and set its version.  T: 64 x kFineTransLd scratch.
+// M's diagonal tile and set its version.  T: 64 x kSmallLd scratch.
 __device__ inline void fine_invert(const FineSweep& w, int b, int k, double* S, double* T, double* aux, double* Mb, int* pivot_flag, int* version, int value) {
   GJOrder order;
   const int n_act = k == w.nt - 1 ? w.last : kSub;
-  const bool singular = gauss_jordan_exchange<kSmallLd, kFineThreads>(S, aux, order, n_act);
+  const bool singular = gauss_jordan_exchange<kSmallLd, kFineThreads>(S, aux, T, order, n_act);
   if (singular && threadIdx.x == 0) report_status(w.status, kDeviceSingularPivot, b, k);
   double* P = w.pinv + ((long long)b * kFinePinv + k % kFinePinv) * kFineTile;
   double* D = Mb + (long long)k * kSub * w.ld + k * kSub;
