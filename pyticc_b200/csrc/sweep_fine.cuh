@@ -64,6 +64,9 @@ struct FineSweep {
 
 __device__ __forceinline__ double* fine_matrix(const FineSweep& w, int b) { return b < w.split ? w.M + (long long)b * w.mstride : w.M2 + (long long)(b - w.split) * w.mstride2; }
 
+// Batch item of matrix b in the device status: its place among its own kind.
+__device__ __forceinline__ int fine_item(const FineSweep& w, int b) { return b < w.split ? b : b - w.split; }
+
 // Positions 0 .. nt - 2 of the block rows other than k, from k + 1 on, cyclic.
 __device__ __forceinline__ int fine_row_at(int k, int nt, int pos) {
   const int j = k + 1 + pos;
@@ -85,7 +88,7 @@ __device__ inline bool fine_wait(const FineSweep& w, const FineNeed& need, int b
     const long long limit = g_step_poll_limit;
     for (long long it = 0;; ++it) {
       if (it >= limit) {
-        if (atomicExch(w.control + 1, 1) == 0) report_status(w.status, kDeviceStalled, b, -1);
+        if (atomicExch(w.control + 1, 1) == 0) report_status(w.status, kDeviceStalled, fine_item(w, b), -1);
         ok = 0;
         break;
       }
@@ -224,7 +227,7 @@ __device__ inline void fine_invert(const FineSweep& w, int b, int k, double* S, 
   GJOrder order;
   const int n_act = k == w.nt - 1 ? w.last : kSub;
   const bool singular = gauss_jordan_exchange<kSmallLd, kFineThreads>(S, aux, T, order, n_act);
-  if (singular && threadIdx.x == 0) report_status(w.status, kDeviceSingularPivot, b, k);
+  if (singular && threadIdx.x == 0) report_status(w.status, kDeviceSingularPivot, fine_item(w, b), k * kSub / kBlock);  // detail: the 128-block, as on the other paths
   double* P = w.pinv + ((long long)b * kFinePinv + k % kFinePinv) * kFineTile;
   double* D = Mb + (long long)k * kSub * w.ld + k * kSub;
   // the inverse out of its exchange order into T (odd row stride: conflict-free columns), then symmetrised on the way out
