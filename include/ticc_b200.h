@@ -7,7 +7,9 @@
  * buffers are caller-owned device pointers; no entry point allocates device
  * memory except the runtime's own one-time module state.  Scratch memory is a
  * caller-provided `workspace` whose size comes from the matching *_workspace_size
- * query.
+ * query.  A workspace that serves a call serves every call whose sizes are none of them
+ * larger; with less than its own query a call may take a slower path (sweeps of a few or
+ * small matrices), whose results differ in rounding.
  *
  * `device_status` (optional, may be NULL) points to int[4] of device memory that
  * the caller zeroes before the call and reads after synchronising the stream:

@@ -49,7 +49,21 @@ struct Carver {
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
-size_t ldmd_layout(ticc::LdmdLayout& L, int n, int n_energy, int n_block, int n_sector, int is_complex, int precision, char* base) {
+// The region of the 64-tile sweeps comes last in a workspace and only where it fits: a size query counts it, a call accepts a
+// workspace without it and then takes 128-wide steps.  What a call cannot do without so grows with every size, which the
+// region does not (use_fine takes a middle batch and leaves a larger one): N = 231 needs 168 MiB for 168 matrices and, with the region, 266
+// for 167.  A workspace sized for the largest of many calls serves them all.
+constexpr size_t kAnySize = ~size_t(0);
+double* take_fine(Carver& c, size_t doubles, size_t available, bool& taken) {
+  Carver with = c;
+  double* p = with.take<double>(doubles);
+  taken = doubles > 0 && with.used + 256 <= available;
+  if (taken) c = with;
+  return taken ? p : nullptr;
+}
+
+// `available`: the workspace's bytes (kAnySize: as many as the fastest path takes; 0: what the call cannot do without).
+size_t ldmd_layout(ticc::LdmdLayout& L, int n, int n_energy, int n_block, int n_sector, int is_complex, int precision, char* base, size_t available) {
   Carver c{base};
   const size_t batch = (size_t)n_block * n_energy;
   L.n = n;
@@ -68,22 +82,24 @@ size_t ldmd_layout(ticc::LdmdLayout& L, int n, int n_energy, int n_block, int n_
   const size_t need_s = ticc::sweep_scratch_doubles(L.npr) * (size_t)(n_sector < 8 ? n_sector : 8);
   L.scratch_doubles = need_e > need_s ? need_e : need_s;
   L.scratch = c.take<double>(L.scratch_doubles);
-  const int used = is_complex ? 2 * n : n;
-  const size_t q_chunk = std::min((size_t)n_sector * n_block, L.scratch_doubles / ticc::sweep_scratch_doubles(L.npr));
-  const bool fine_m = precision == TICC_PRECISION_FP64 && ticc::use_fine(used, batch), fine_q = ticc::use_fine(n, q_chunk);
-  const size_t q_count = (size_t)n_sector * n_block;
-  L.joint_q = ticc::ldmd_joint_qmid(n, batch, q_count, is_complex, precision == TICC_PRECISION_FP64);
-  const size_t fine = std::max(fine_m ? ticc::fine_total_doubles(ticc::fine_tiles(used), batch + (L.joint_q ? q_count : 0)) : 0, fine_q ? ticc::fine_total_doubles(ticc::fine_tiles(n), q_chunk) : 0);
-  double* fine_base = fine > 0 ? c.take<double>(fine) : nullptr;
-  L.fine = fine_m ? fine_base : nullptr;
-  L.fine_q = fine_q ? fine_base : nullptr;
   L.reduced = (precision == TICC_PRECISION_MIXED) ? c.take<int>((size_t)n_sector) : nullptr;
   L.split = (precision == TICC_PRECISION_MIXED) ? c.take<float>(ticc::tc_split_floats(L.np, (int)batch)) : nullptr;
   if (base == nullptr) L.reduced = nullptr, L.split = nullptr;
+  const int used = is_complex ? 2 * n : n;
+  const size_t q_chunk = std::min((size_t)n_sector * n_block, L.scratch_doubles / ticc::sweep_scratch_doubles(L.npr));
+  const size_t q_count = (size_t)n_sector * n_block;
+  const bool fine_m = precision == TICC_PRECISION_FP64 && ticc::use_fine(used, batch), fine_q = ticc::use_fine(n, q_chunk);
+  const bool joint = ticc::ldmd_joint_qmid(n, batch, q_count, is_complex, precision == TICC_PRECISION_FP64);
+  const size_t fine = std::max(fine_m ? ticc::fine_total_doubles(ticc::fine_tiles(used), batch + (joint ? q_count : 0)) : 0, fine_q ? ticc::fine_total_doubles(ticc::fine_tiles(n), q_chunk) : 0);
+  bool taken;
+  double* fine_base = take_fine(c, fine, available, taken);
+  L.fine = fine_m ? fine_base : nullptr;
+  L.fine_q = fine_q ? fine_base : nullptr;
+  L.joint_q = joint && taken;
   return c.used + 256;
 }
 
-size_t match_layout(ticc::MatchLayout& L, int n, int n_energy, int is_complex, int max_open, char* base) {
+size_t match_layout(ticc::MatchLayout& L, int n, int n_energy, int is_complex, int max_open, char* base, size_t available) {
   Carver c{base};
   L.n = n;
   L.n_energy = n_energy;
@@ -104,7 +120,8 @@ size_t match_layout(ticc::MatchLayout& L, int n, int n_energy, int is_complex, i
   const int np = L.npz > L.npa ? L.npz : L.npa;
   L.scratch = c.take<double>((size_t)n_energy * ticc::sweep_scratch_doubles(np));
   const int used = is_complex ? 2 * n : n;
-  L.fine = ticc::use_fine(used, n_energy) ? c.take<double>(ticc::fine_total_doubles(ticc::fine_tiles(used), n_energy)) : nullptr;
+  bool taken;
+  L.fine = take_fine(c, ticc::use_fine(used, n_energy) ? ticc::fine_total_doubles(ticc::fine_tiles(used), n_energy) : 0, available, taken);
   return c.used + 256;
 }
 
@@ -126,20 +143,21 @@ int ticc_last_error(char* buf, size_t len) {
 }
 
 // ---- symmetric inversion ---------------------------------------------------------------
-static size_t sym_layout(int n, int batch, int is_complex, double** M, double** scratch, char* base, double** fine = nullptr) {
+static size_t sym_layout(int n, int batch, int is_complex, double** M, double** scratch, char* base, size_t available = 0, double** fine = nullptr) {
   Carver c{base};
   const int np = ticc::ldmd_np(n, is_complex);
   *M = c.take<double>((size_t)batch * np * np);
   *scratch = c.take<double>((size_t)batch * ticc::sweep_scratch_doubles(np));
   const int used = is_complex ? 2 * n : n;
-  if (fine != nullptr) *fine = ticc::use_fine(used, batch) ? c.take<double>(ticc::fine_total_doubles(ticc::fine_tiles(used), batch)) : nullptr;
+  bool taken;
+  if (fine != nullptr) *fine = take_fine(c, ticc::use_fine(used, batch) ? ticc::fine_total_doubles(ticc::fine_tiles(used), batch) : 0, available, taken);
   return c.used + 256;
 }
 
 int ticc_sym_inverse_workspace_size(int n, int batch, int is_complex, size_t* bytes) {
   if (n < 1 || batch < 1 || bytes == nullptr) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_sym_inverse_workspace_size: n=%d batch=%d", n, batch);
   double *M, *s, *fine;
-  *bytes = sym_layout(n, batch, is_complex, &M, &s, nullptr, &fine);
+  *bytes = sym_layout(n, batch, is_complex, &M, &s, nullptr, kAnySize, &fine);
   return TICC_OK;
 }
 
@@ -190,9 +208,9 @@ __global__ void sym_store_kernel(const double* M, int np, double* dst, int n, in
 int ticc_sym_inverse(void* M, int n, int batch, int is_complex, void* workspace, size_t workspace_bytes, int* device_status, void* stream) {
   if (M == nullptr || n < 1 || batch < 1) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_sym_inverse: M=%p n=%d batch=%d", M, n, batch);
   double *Mw, *scratch, *fine;
-  const size_t need = sym_layout(n, batch, is_complex, &Mw, &scratch, nullptr, &fine);
+  const size_t need = sym_layout(n, batch, is_complex, &Mw, &scratch, nullptr);
   if (workspace == nullptr || workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "ticc_sym_inverse: workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-  sym_layout(n, batch, is_complex, &Mw, &scratch, static_cast<char*>(workspace), &fine);
+  sym_layout(n, batch, is_complex, &Mw, &scratch, static_cast<char*>(workspace), workspace_bytes, &fine);
   ticc::FineState state{fine};
   const int np = ticc::ldmd_np(n, is_complex);
   const long long nl = is_complex ? np / 2 : np;
@@ -228,9 +246,9 @@ static int ldmd_run(const char* who, void* Y, int is_complex, const double* ener
   if (rc != TICC_OK) return rc;
   if (!(reduced_mass > 0.0)) return fail(TICC_ERR_INVALID_ARGUMENT, "%s: reduced_mass must be positive, got %g", who, reduced_mass);
   ticc::LdmdLayout L{};
-  const size_t need = ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, nullptr);
+  const size_t need = ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, nullptr, 0);
   if (workspace == nullptr || workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "%s: workspace of %zu bytes given, %zu needed", who, workspace_bytes, need);
-  ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, static_cast<char*>(workspace));
+  ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, static_cast<char*>(workspace), workspace_bytes);
   ticc::LdmdSectors sec{half_steps, W_start, W_mid, W_end, W_start_stride, W_mid_stride, W_end_stride, n_sector, W_block_stride};
   cudaError_t e = ticc::ldmd_propagate(static_cast<double*>(Y), energies, reduced_mass, sec, L, device_status, as_stream(stream));
   return e == cudaSuccess ? TICC_OK : cuda_fail(e, who);
@@ -241,7 +259,7 @@ int ticc_ldmd_workspace_size(int n_channel, int n_energy, int n_sector, int is_c
   const int rc = ldmd_check_sizes("ticc_ldmd_workspace_size", n_channel, n_energy, 1, n_sector, precision);
   if (rc != TICC_OK) return rc;
   ticc::LdmdLayout L{};
-  *bytes = ldmd_layout(L, n_channel, n_energy, 1, n_sector, is_complex, precision, nullptr);
+  *bytes = ldmd_layout(L, n_channel, n_energy, 1, n_sector, is_complex, precision, nullptr, kAnySize);
   return TICC_OK;
 }
 
@@ -259,9 +277,9 @@ int ticc_ldmd_reduced_blocks(const void* workspace, size_t workspace_bytes, int 
   if (rc != TICC_OK) return rc;
   if (precision != TICC_PRECISION_MIXED) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_ldmd_reduced_blocks: only mixed-precision calls reduce sweep blocks");
   ticc::LdmdLayout L{};
-  const size_t need = ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, nullptr);
+  const size_t need = ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, nullptr, 0);
   if (workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "ticc_ldmd_reduced_blocks: workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-  ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, static_cast<char*>(const_cast<void*>(workspace)));
+  ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, static_cast<char*>(const_cast<void*>(workspace)), workspace_bytes);
   const cudaError_t e = cudaMemcpyAsync(counts, L.reduced, sizeof(int) * (size_t)n_sector, cudaMemcpyDeviceToHost, as_stream(stream));
   return e == cudaSuccess ? TICC_OK : cuda_fail(e, "ticc_ldmd_reduced_blocks");
 }
@@ -271,7 +289,7 @@ int ticc_ldmd_blocks_workspace_size(int n_channel, int n_energy, int n_block, in
   const int rc = ldmd_check_sizes("ticc_ldmd_blocks_workspace_size", n_channel, n_energy, n_block, n_sector, precision);
   if (rc != TICC_OK) return rc;
   ticc::LdmdLayout L{};
-  *bytes = ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, nullptr);
+  *bytes = ldmd_layout(L, n_channel, n_energy, n_block, n_sector, is_complex, precision, nullptr, kAnySize);
   return TICC_OK;
 }
 
@@ -490,7 +508,7 @@ int ticc_match_workspace_size(int n_channel, int n_energy, int is_complex, int m
   if (n_channel < 1 || n_energy < 1 || max_open < 0 || max_open > n_channel || bytes == nullptr)
     return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_match_workspace_size: n_channel=%d n_energy=%d max_open=%d", n_channel, n_energy, max_open);
   ticc::MatchLayout L{};
-  *bytes = match_layout(L, n_channel, n_energy, is_complex, max_open, nullptr);
+  *bytes = match_layout(L, n_channel, n_energy, is_complex, max_open, nullptr, kAnySize);
   return TICC_OK;
 }
 
@@ -503,9 +521,9 @@ int ticc_match_smatrix(const void* Y, int is_complex, double Rmatch, const doubl
   if (!(Rmatch > 0.0) || !(reduced_mass > 0.0))
     return fail(TICC_ERR_INVALID_ARGUMENT, "Rmatch and reduced_mass must be positive, but got Rmatch=%g, reduced_mass=%g", Rmatch, reduced_mass);
   ticc::MatchLayout Lay{};
-  const size_t need = match_layout(Lay, n_channel, n_energy, is_complex, max_open, nullptr);
+  const size_t need = match_layout(Lay, n_channel, n_energy, is_complex, max_open, nullptr, 0);
   if (workspace == nullptr || workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "ticc_match_smatrix: workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-  match_layout(Lay, n_channel, n_energy, is_complex, max_open, static_cast<char*>(workspace));
+  match_layout(Lay, n_channel, n_energy, is_complex, max_open, static_cast<char*>(workspace), workspace_bytes);
   cudaError_t e = ticc::match_smatrix(static_cast<const double*>(Y), Rmatch, energies, reduced_mass, E_int, L, S, n_open, Lay, device_status, as_stream(stream));
   return e == cudaSuccess ? TICC_OK : cuda_fail(e, "ticc_match_smatrix");
 }
