@@ -446,7 +446,7 @@ __device__ inline bool small_sweep_then(double* S, double* aux, int used, P&& pr
       w[u] = (D == 32 && r < used && c <= r) ? pre(r, c) : 0.0;  // (64 rows: the registers are the exchange's)
     }
     GJOrder order;
-    const bool singular = gauss_jordan_exchange<Sh::kLd, Sh::kThreads, D>(S, aux, aux + kGJAuxDoubles, order, n_act);
+    const bool singular = gauss_jordan_exchange<Sh::kLd, Sh::kThreads, D>(S, aux, order, n_act, GJFromCopy<Sh::kLd, Sh::kThreads, D>{aux + kGJAuxDoubles});
 #pragma unroll
     for (int u = 0; u < Sh::kPer; ++u) {
       const int e = threadIdx.x + u * Sh::kThreads, r = e / D, c = e % D;

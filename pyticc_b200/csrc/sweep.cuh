@@ -173,35 +173,17 @@ __device__ __forceinline__ unsigned long long gj_factor_panel(const double* src,
   return all & ~rows_before;
 }
 
-// Copy of a strip in the order of its registers (D x D doubles in all): conflict-free (at row stride D + 4 the copy cost 1 % of a sweep).
-template <int D>
-__device__ __forceinline__ void gj_save_strip(const GJStrip<D>& g, double* save) {
-#pragma unroll
-  for (int mt = 0; mt < D / 8; ++mt) reinterpret_cast<double2*>(save)[((threadIdx.x >> 5) * (D / 8) + mt) * 32 + (threadIdx.x & 31)] = g.v[mt];
-}
-template <int D>
-__device__ __forceinline__ double gj_saved(const double* save, int r, int c) {
-  return save[2 * (((c >> 3) * (D / 8) + (r >> 3)) * 32 + (r & 7) * 4 + ((c & 7) >> 1)) + (c & 1)];
-}
-
-// The exchange below, column by column, from the copy of the block in `save`: for blocks with a pivot that is
-// subnormal, 2^1021 or more, or not finite.  Pivot: the largest magnitude (a NaN above all), the smallest row on ties; its
-// reciprocal is formed at a scale where both are normal.  Returns true if a pivot was zero or non-finite.
+// The exchange below, column by column, of the block in S: for blocks with a pivot that is subnormal, 2^1021 or more, or not
+// finite.  Pivot: the largest magnitude (a NaN above all), the smallest row on ties; its reciprocal is formed at a scale
+// where both are normal.  Returns true if a pivot was zero or non-finite.
 // Inlined behind the fast exchange's last barrier and without a divide operator: a call anywhere in the kernel, or a branch to
-// the careful way inside a panel, slowed the fast exchange (N = 1000: 382 -> 406 us a sweep; as it stands 384, the
-// copy of the block being most of it).
+// the careful way inside a panel, slowed the fast exchange (N = 1000: 382 -> 406 us a sweep).
 template <int Ld, int kThreads, int D>
-__device__ __forceinline__ bool gauss_jordan_any_range(double* S, const double* save, int* perm, int n_act) {
+__device__ __forceinline__ bool gauss_jordan_any_range(double* S, int* perm, int n_act) {
   constexpr int kPer = D * D / kThreads;
   const int t = threadIdx.x, lane = t & 31;
   bool singular = false;
   unsigned long long used = n_act == 64 ? 0ull : ~0ull << n_act;
-#pragma unroll 1
-  for (int u = 0; u < kPer; ++u) {
-    const int e = t + u * kThreads, r = e / D, c = e % D;
-    S[r * Ld + c] = gj_saved<D>(save, r, c);
-  }
-  __syncthreads();
 #pragma unroll 1
   for (int j = 0; j < n_act; ++j) {
     // every warp finds the pivot for itself; rank: 1 + the magnitude's bits, 0 for a used row
@@ -241,8 +223,9 @@ __device__ __forceinline__ bool gauss_jordan_any_range(double* S, const double* 
 
 // S <- S^{-1} (D x D in shared memory, D = 32 or 64, row stride Ld = 4 mod 16) by Gauss-Jordan exchange with partial pivoting over
 // the block's rows, by the kThreads threads of the CTA.  `n_act` (a multiple of kGJPanel): rows and columns at or beyond
-// it hold the identity and are left alone.  `save` (D x D): scratch, receives a copy of the block beside the first
-// panel's elimination.  Returns true if a pivot was zero or non-finite.  Uses named barrier 1.
+// it hold the identity and are left alone.  `again`: what brings the block back into S
+// for gauss_jordan_any_range, its object told each strip first.  Returns true if a pivot was zero or non-finite.  Uses
+// named barrier 1.
 //
 // The exchange of one column is a serial chain (rank the rows, reciprocal, publish the row, update), so the work around
 // that chain is what costs.  It is blocked: one warp eliminates a panel of 8 columns in registers, with no barrier, no
@@ -260,8 +243,8 @@ struct GJOrder {
   const int* perm;
   const int* iperm;
 };
-template <int Ld, int kThreads, int D = kSub>
-__device__ inline bool gauss_jordan_exchange(double* S, double* aux, double* save, GJOrder& order, int n_act = D) {
+template <int Ld, int kThreads, int D = kSub, class Again>
+__device__ inline bool gauss_jordan_exchange(double* S, double* aux, GJOrder& order, int n_act, const Again& again) {
   static_assert(kThreads / 32 == D / kGJPanel, "a strip for every warp");
   constexpr int kWarps = kThreads / 32, kTiles = D / 8 / 4;  // row tiles of the next panel that each of its four warps updates
   unsigned long long* panel_rows = reinterpret_cast<unsigned long long*>(aux);  // [kSub / kGJPanel]
@@ -275,7 +258,7 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, double* sav
   if (t >= n_act && t < D) perm[t] = t;
   GJStrip<D> g;
   gj_load_strip<Ld, D>(g, S, kGJPanel * warp);
-  gj_save_strip<D>(g, save);
+  again.keep(g);
   __syncwarp();
   if (warp == 0) {
     const unsigned long long m = gj_factor_panel<Ld, D>(S, Ld, S, perm, 0, used, outside);
@@ -328,16 +311,35 @@ __device__ inline bool gauss_jordan_exchange(double* S, double* aux, double* sav
   order.iperm = iperm;
   bool singular = false;
   if (__syncthreads_or(outside)) {
-    singular = gauss_jordan_any_range<Ld, kThreads, D>(S, save, perm, n_act);
+    again.restore(S);
+    singular = gauss_jordan_any_range<Ld, kThreads, D>(S, perm, n_act);
     if (t < D) iperm[perm[t]] = t;
     __syncthreads();
   }
   return singular;
 }
+// From a copy in `save` (D x D doubles), which is written beside the first panel's elimination, in the order of the strips'
+// registers: conflict-free (row by row it cost 1 % of a sweep, so 0.5 %).
+template <int Ld, int kThreads, int D>
+struct GJFromCopy {
+  double* save;
+  __device__ __forceinline__ void keep(const GJStrip<D>& g) const {
+#pragma unroll
+    for (int mt = 0; mt < D / 8; ++mt) reinterpret_cast<double2*>(save)[((threadIdx.x >> 5) * (D / 8) + mt) * 32 + (threadIdx.x & 31)] = g.v[mt];
+  }
+  __device__ __forceinline__ void restore(double* S) const {
+#pragma unroll 1
+    for (int e = threadIdx.x; e < D * D; e += kThreads) {
+      const int r = e / D, c = e % D;
+      S[r * Ld + c] = save[2 * (((c >> 3) * (D / 8) + (r >> 3)) * 32 + (r & 7) * 4 + ((c & 7) >> 1)) + (c & 1)];
+    }
+    __syncthreads();
+  }
+};
 template <int Ld, int kThreads>
 __device__ inline bool gauss_jordan_sub(double* S, double* aux, double* save, int n_act = kSub) {
   GJOrder order;
-  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, save, order, n_act);
+  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, order, n_act, GJFromCopy<Ld, kThreads, kSub>{save});
   constexpr int kPer = kSub * kSub / kThreads;
   double x[kPer];
 #pragma unroll

@@ -221,12 +221,39 @@ __device__ __forceinline__ void fine_each(FineAcc& acc, F&& f) {
 // writes the transpose.
 __device__ __forceinline__ bool fine_mirrors(int ta, int tb, bool last) { return last && ta == tb + 1 && (tb & 1) == 0; }
 
+// A pivot block once more, for gauss_jordan_any_range, from what it was made of: M's diagonal tile, which is written after the
+// inversion only, less X R^T behind a panel (X in its slot, which no step after the next writes before this
+// block's pivot is out, and R in shared memory).  Nothing to keep, and no pointer of its own: the kernel with two CTAs an
+// SM has no register for one (2 % of a sweep).
+struct FineAgain {
+  const FineSweep& w;
+  int b, k;
+  const double* R;
+  __device__ __forceinline__ void keep(const GJStrip<kSub>&) const {}
+  __device__ __forceinline__ void restore(double* S) const {
+    const double* C = fine_matrix(w, b) + (long long)k * kSub * w.ld + k * kSub;
+    const double* X = w.slots + (((long long)b * kFineSlots + (k - 1) % kFineSlots) * 2 * w.nt + k) * kFineTile;
+#pragma unroll 1
+    for (int e = threadIdx.x; e < kFineTile; e += kFineThreads) {  // the lower half to both places
+      const int r = e / kSub, c = e % kSub, i = max(r, c), j = min(r, c);
+      double v = __ldcg(C + (long long)i * w.ld + j);
+      if (k > 0) {
+#pragma unroll 1
+        for (int q = 0; q < kSub; ++q) v = fma(-__ldcg(X + i * kSub + q), R[j * kSmallLd + q], v);
+      }
+      S[r * kSmallLd + c] = v;
+    }
+    __syncthreads();
+  }
+};
+
 // Invert the symmetric block in S; publish P^{-1} first (`pivot_flag`, on which the chain waits), then write -P^{-1} into
-// M's diagonal tile and set its version.  T: 64 x kSmallLd scratch.
+// M's diagonal tile and set its version.  T: 64 x kFineTransLd scratch, written after the inversion
+// (behind a panel it comes with R, row stride kSmallLd).
 __device__ inline void fine_invert(const FineSweep& w, int b, int k, double* S, double* T, double* aux, double* Mb, int* pivot_flag, int* version, int value) {
   GJOrder order;
   const int n_act = k == w.nt - 1 ? w.last : kSub;
-  const bool singular = gauss_jordan_exchange<kSmallLd, kFineThreads>(S, aux, T, order, n_act);
+  const bool singular = gauss_jordan_exchange<kSmallLd, kFineThreads>(S, aux, order, n_act, FineAgain{w, b, k, T});
   if (singular && threadIdx.x == 0) report_status(w.status, kDeviceSingularPivot, fine_item(w, b), k * kSub / kBlock);  // detail: the 128-block, as on the other paths
   double* P = w.pinv + ((long long)b * kFinePinv + k % kFinePinv) * kFineTile;
   double* D = Mb + (long long)k * kSub * w.ld + k * kSub;

@@ -24,9 +24,10 @@ def test_one_channel_from_the_subnormals_to_the_top():
     assert (np.abs(X - want) <= np.maximum(2.0**-52 * np.abs(want), 2.0**-1074)).all()
 
 
+# 150 x 128 and 330: the 64-tile sweep with two CTAs an SM, and with more steps than slots
 @pytest.mark.parametrize("exponent", [-1023, -1021, 1019, 1020, 1021])
-@pytest.mark.parametrize("n", [9, 40, 150])
-def test_scaled_matrices(n, exponent):
+@pytest.mark.parametrize("n,batch", [(9, 1), (40, 1), (100, 1), (150, 1), (150, 128), (330, 2)])
+def test_scaled_matrices(n, batch, exponent):
     """A = 2^exponent (D + small): diagonal 1.5 to 1.9 and weak couplings, both exact at every scale.  The inverse is that of
     the unscaled matrix times 2^-exponent; its elements carry at most the rounding of 51-bit (subnormal) numbers per
     elimination step, and an absolute unit 2^-1074 where the inverse itself is subnormal."""
@@ -34,7 +35,9 @@ def test_scaled_matrices(n, exponent):
     noise = np.round(rng.uniform(-1.0, 1.0, (n, n)) * 0.02 / np.sqrt(n) * 2.0**20) * 2.0**-20
     A = np.tril(noise, -1)
     A = A + A.T + np.diag(np.round(rng.uniform(1.5, 1.9, n) * 2.0**20) * 2.0**-20)
-    X = _sym_inverse(np.ldexp(A, exponent)[None], False)[0]
+    X = _sym_inverse(np.repeat(np.ldexp(A, exponent)[None], batch, axis=0), False)
+    np.testing.assert_array_equal(X, np.repeat(X[:1], batch, axis=0))
+    X = X[0]
     # compared at the scale of the unscaled inverse, in two exact steps
     X = np.ldexp(np.ldexp(X, exponent // 2), exponent - exponent // 2)
     np.testing.assert_allclose(X, np.linalg.inv(A), rtol=0, atol=4 * n * (2.0**-51 + 2.0 ** (exponent - 1074)))
