@@ -218,9 +218,11 @@ inline cudaError_t contract_groups_by(const ContractTiles& tiles, const double* 
   }
   return e;
 }
-// How many radial points share a CTA: as many as leave the six CTAs that an SM holds (five for four points) some two to three times over.
-// Measured, us a call, 1 / 2 / 4 points (units: tiles x radial points): AB+CD pair, 579 tiles, 2316 units 1205 / 1066 / 1011,
-// 4632 2287 / 1949 / 1867, 13896 6613 / 5573 / 5301; vibrating A+BC, 150 tiles, 1350 units 238 / 273 / 289, 2550 353 / 358 /
+// How many radial points share a CTA.  Sharing saves the rows' copies and costs CTAs, which long grids bear better than short
+// ones, so the lines lie between the two systems measured: two points from 2200 units (tiles x radial points) on, 1100
+// CTAs for the 888 places of 148 SMs (six each), four from 4600 on, 1150 CTAs for 740 places (five each).
+// Measured, us a call, 1 / 2 / 4 points: AB+CD pair (2 x 2700 grid points), 579 tiles, 2316 units 1205 / 1066 / 1011,
+// 4632 2287 / 1949 / 1867, 13896 6613 / 5573 / 5301; vibrating A+BC (1024), 150 tiles, 1350 units 238 / 273 / 289, 2550 353 / 358 /
 // 374, 4950 628 / 605 / 606, 13500 1608 / 1483 / 1387.
 inline cudaError_t contract_groups(const ContractTiles& tiles, const double* Br, const double* Bi, const int* row_out, int n_grid, double scale, const double* potential, long long pot_stride, int n_R,
                                    int n, double* out, cudaStream_t stream) {

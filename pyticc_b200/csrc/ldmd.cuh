@@ -223,8 +223,9 @@ __global__ void __launch_bounds__(kElemThreads) ldmd_elementwise_kernel(int s, i
   const int n = L.n, np = L.np, ne = L.n_energy, batch = L.n_block * ne;
   const int i0 = ta * kCols + (blockIdx.x % kGroups) * kElemRows, j0 = tb * kCols;
   const int e0 = blockIdx.y * e_per, e1 = min(ne, e0 + e_per);
-  // The W matrices, y1, y2 and (but for the first sector) Q_mid were complete before the sweep ahead of this pass began:
-  // their part is read while that sweep drains.
+  // The W matrices and (but for the first sector) Q_mid were complete before the sweep ahead of this pass began: their part is
+  // read ahead of the wait.  A sweep does not let its successor start before its last CTA has left, so for a pass that is
+  // its launch and these loads; the sweep behind a pass comes up with the pass's last wave.
   next_kernel_may_start();
   if (s == 0) previous_kernel_done();
   if (kPhase == 3 && i0 >= n) return;

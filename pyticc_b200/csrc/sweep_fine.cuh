@@ -509,8 +509,9 @@ inline cudaError_t fine_sweep(FineState& state, double* M, long long mstride, in
   w.base = state.sweeps * nt;
   w.queue_base = state.queue;
   // One CTA per SM leaves the chain its SM (and twice the registers); two where a step has more units than four waves of
-  // that.  Measured, us a sweep, one / two per SM: N = 231, batch 32 (288 units a step) 119 / 139, batch 64 (576) 156 / 145;
-  // N = 660, batch 8 (520) 318 / 356, batch 16 (1040) 574 / 424; N = 1984, batch 1 (495) 809 / 983, batch 4 2876 / 2063.
+  // that.  Measured, us an inversion call (its loads and stores included), one / two per SM: N = 231, batch 32 (288 units a
+  // step) 139 / 156, batch 64 (576) 205 / 188; N = 512, batch 16 (560) 306 / 306; N = 660, batch 8 (520) 370 / 375, batch 16
+  // (1040) 650 / 519; N = 1984, batch 1 (495) 894 / 944, batch 2 (990) 1487 / 1150; N = 2610, batch 1 (860) 1779 / 1482.
   const bool dense = (long long)batch * (t + t * (t + 1) / 2) > 4LL * sms;
   const long long slots = dense ? 2LL * sms : sms;
   const int grid = (int)(total < slots ? total : slots);
@@ -531,10 +532,14 @@ inline cudaError_t sweep_any(FineState& fine, double* M, long long mstride, int 
 
 // Whether a batch of FP64 sweeps of n_used rows takes the 64-tile path: where its estimated time is below that of the
 // 128-tile steps, both the larger of a latency (per step of the chain) and a throughput (per cubed tile count) term, in
-// us.  Measured, us a sweep, 128-tile steps / here: N = 192, batch 16: 221 / 76; N = 231, batch 16: 221 / 98, batch 128: 241 / 207;
-// N = 396, batch 8: 442 / 166; N = 512, batch 32: 484 / 324, batch 64: 622 / 672; N = 660, batch 4: 664 / 255, batch 64: 1728 / 1688;
-// N = 1024, batch 8: 925 / 594, batch 16: 1157 / 1206; N = 1984, batch 1: 1772 / 760, batch 8: 3524 / 4230; N = 100 (one
-// 128 block, no steps): 50 / 53.
+// us.  (The chain's 28 us a link is a large matrix's, 23 at N = 660; it never decides, a 128-step costing four times as
+// much.)  An odd tile count saves the steps' padding, so that up to nine tiles every batch comes here.
+// Measured, us an inversion call (its loads and stores included), 128-tile steps / here: N = 192, batch 16 229 / 101, 128 321 / 199,
+// 1000 2081 / 1302; N = 231, 16 232 / 120, 128 334 / 304, 200 534 / 460 (left to the steps); N = 320, 128 771 / 562, 1000
+// 5315 / 4230; N = 396, 8 442 / 195, 64 766 / 616; N = 448, 1000 10722 / 9574; N = 512, 32 573 / 436, 64 809 / 871; N = 576,
+// 128 2527 / 2411, 1000 18829 / 18847; N = 660, 4 649 / 286, 16 772 / 519, 64 2062 / 2035 (left); N = 1024, 8 977 / 700, 16
+// 1327 / 1403; N = 1984, 1 1685 / 896, 2 1772 / 1148, 4 2330 / 2174 (left), 8 3744 / 4514; N = 2610, 1 2256 / 1482, 2 2468 /
+// 2364 (left).
 inline bool use_fine(int n_used, size_t batch) {
   const int nt = fine_tiles(n_used), steps = (n_used + kBlock - 1) / kBlock;
   if (steps < 2 || nt > kFineMaxTiles) return false;

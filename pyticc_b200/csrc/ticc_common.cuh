@@ -47,7 +47,8 @@ inline void note_launch(long long n = 1) { launch_counter().fetch_add(n, std::me
 // Launch `kernel` so that its CTAs may come up while the kernel before it in the stream drains: the CTAs of a kernel launched so
 // call previous_kernel_done() before they touch anything that the call's earlier kernels write.  A kernel that starts
 // behind such a one and waits is ordered behind everything before it too, because the other finished only after its own wait.
-// Between the passes and sweeps of a propagation this hides the launch, the first loads and a sweep's thinning tail:
+// Between the passes and sweeps of a propagation this hides the launch and the first loads (only the passes call
+// next_kernel_may_start(), so nothing runs beside a sweep's thinning tail):
 // measured, N = 231, 16 energies, 8 sectors 1865 -> 1808 us, a rigid-rotor solve of 24 sectors 7.96 -> 7.69 ms, mixed windows of N = 1860 24.7 -> 24.5 ms.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
