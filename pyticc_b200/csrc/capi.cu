@@ -414,13 +414,15 @@ int ticc_pes_legendre_grid(const double* R, int n_R, const double* r, int n_r, c
 }
 
 // ---- BF -> SF transform ------------------------------------------------------------------------------
-static size_t transform_layout(int n, int batch, double** Bp, double** P, double** T, int** lists, char* base) {
+// flags: 4 (of each part, Y's plane and its first product: a value that is not finite), then B's chunks with non-zeros
+static size_t transform_layout(int n, int batch, double** Bp, double** P, double** T, int** flags, size_t* n_flags, char* base) {
   Carver c{base};
   const int np = ticc::ldmd_np(n, 0);
   *Bp = c.take<double>((size_t)np * np);
   *P = c.take<double>((size_t)batch * np * np);
   *T = c.take<double>((size_t)batch * np * np);
-  *lists = c.take<int>(4 + (size_t)(np / ticc::kBlock) * (np / ticc::kChunk + 1));  // non-finite flag, chunk lists
+  *n_flags = 4 + (size_t)(np / ticc::kBlock) * (np / ticc::kChunk);
+  *flags = c.take<int>(*n_flags);
   return c.used + 256;
 }
 
@@ -428,40 +430,40 @@ int ticc_transform_workspace_size(int n, int batch, int is_complex, size_t* byte
   if (n < 1 || batch < 1 || bytes == nullptr) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_transform_workspace_size: n=%d batch=%d", n, batch);
   double *a, *b, *c;
   int* d;
-  *bytes = transform_layout(n, batch, &a, &b, &c, &d, nullptr);
+  size_t n_flags;
+  *bytes = transform_layout(n, batch, &a, &b, &c, &d, &n_flags, nullptr);
   return TICC_OK;
 }
 
 int ticc_transform_bf_to_sf(const void* Y, void* Y_out, const double* B, int n, int batch, int is_complex, void* workspace, size_t workspace_bytes, void* stream) {
   if (Y == nullptr || Y_out == nullptr || B == nullptr || n < 1 || batch < 1) return fail(TICC_ERR_INVALID_ARGUMENT, "ticc_transform_bf_to_sf: bad arguments");
   double *Bp, *P, *T;
-  int* flag;
-  const size_t need = transform_layout(n, batch, &Bp, &P, &T, &flag, nullptr);
+  int* flags;
+  size_t n_flags;
+  const size_t need = transform_layout(n, batch, &Bp, &P, &T, &flags, &n_flags, nullptr);
   if (workspace == nullptr || workspace_bytes < need) return fail(TICC_ERR_WORKSPACE, "ticc_transform_bf_to_sf: workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-  transform_layout(n, batch, &Bp, &P, &T, &flag, static_cast<char*>(workspace));
-  int* lists = flag + 4;
+  transform_layout(n, batch, &Bp, &P, &T, &flags, &n_flags, static_cast<char*>(workspace));
+  int* has = flags + 4;
   const int np = ticc::ldmd_np(n, 0);
   cudaStream_t s = as_stream(stream);
   const long long area = (long long)np * np;
-  ticc::pad_plane_kernel<<<dim3(ticc::grid_for(area, 256, 8192), 1), 256, 0, s>>>(B, n, 0, 0, Bp, np);
+  cudaError_t e = cudaSuccess;
+  ticc::pad_chunks_kernel<<<(unsigned)(n_flags - 4), ticc::kPadThreads, 0, s>>>(B, n, Bp, np, has, flags, 4);
   ticc::note_launch();
   for (int part = 0; part < (is_complex ? 2 : 1); ++part) {
-    cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
-    if (e != cudaSuccess) return cuda_fail(e, "ticc_transform_bf_to_sf");
+    int* flag = flags + 2 * part;
     ticc::pad_plane_kernel<<<dim3(ticc::grid_for(area, 256, 8192), batch), 256, 0, s>>>(static_cast<const double*>(Y), n, is_complex, part, P, np, flag);
     ticc::note_launch();
     // T^T = (B^T Y)^T, then (B^T T^T)^T = T B = B^T Y B, over the row chunks of B that hold non-zeros
     for (int half = 0; half < 2; ++half) {
-      ticc::chunk_list_kernel<<<np / ticc::kBlock, ticc::kListThreads, 0, s>>>(Bp, np, np, flag, lists);
-      ticc::note_launch();
-      const ticc::GemmBatch g{Bp, np, 0, half == 0 ? P : T, np, area, half == 0 ? T : P, np, area, np, 1.0, 1, lists, flag};
+      const ticc::GemmBatch g{Bp, np, 0, half == 0 ? P : T, np, area, half == 0 ? T : P, np, area, np, 1.0, 1, has, flag, 1 + half, half == 0 ? flag + 1 : nullptr};
       e = ticc::gemm_tn(g, np, np, batch, s);
       if (e != cudaSuccess) return cuda_fail(e, "ticc_transform_bf_to_sf");
     }
     ticc::unpad_plane_kernel<<<dim3(ticc::grid_for((long long)n * n, 256, 8192), batch), 256, 0, s>>>(P, np, static_cast<double*>(Y_out), n, is_complex, part);
     ticc::note_launch();
   }
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? TICC_OK : cuda_fail(e, "ticc_transform_bf_to_sf");
 }
 

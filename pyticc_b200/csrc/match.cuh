@@ -214,7 +214,7 @@ inline cudaError_t match_smatrix(const double* Y, double Rmatch, const double* e
   const int used = 2 * L.max_open;
   err = sweep_general(L.A, (long long)L.npa * L.npa, L.npa, L.n_energy, L.scratch, status, stream, used);
   if (err != cudaSuccess) return err;
-  GemmBatch g{L.A, L.npa, (long long)L.npa * L.npa, L.B, L.npa, (long long)L.npa * L.npa, L.C, L.npa, (long long)L.npa * L.npa, (int)round_up(used > 0 ? used : 1, kChunk), 1.0, 0, nullptr, nullptr};
+  GemmBatch g{L.A, L.npa, (long long)L.npa * L.npa, L.B, L.npa, (long long)L.npa * L.npa, L.C, L.npa, (long long)L.npa * L.npa, (int)round_up(used > 0 ? used : 1, kChunk), 1.0, 0, nullptr, nullptr, 0, nullptr};
   err = gemm_tn(g, L.npa, L.npa, L.n_energy, stream);
   if (err != cudaSuccess) return err;
   match_extract_kernel<<<dim3(grid_for((long long)L.n * L.n, 256, 8192), L.n_energy), 256, 0, stream>>>(L, n_open, S, status);
