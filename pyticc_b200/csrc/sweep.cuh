@@ -336,10 +336,22 @@ struct GJFromCopy {
     __syncthreads();
   }
 };
+// From where the block was read (row stride ld), still there.
 template <int Ld, int kThreads>
-__device__ inline bool gauss_jordan_sub(double* S, double* aux, double* save, int n_act = kSub) {
+struct GJFromSource {
+  const double* source;
+  long long ld;
+  __device__ __forceinline__ void keep(const GJStrip<kSub>&) const {}
+  __device__ __forceinline__ void restore(double* S) const {
+#pragma unroll 1
+    for (int e = threadIdx.x; e < kSub * kSub; e += kThreads) S[(e / kSub) * Ld + e % kSub] = source[(e / kSub) * ld + e % kSub];
+    __syncthreads();
+  }
+};
+template <int Ld, int kThreads, class Again>
+__device__ inline bool gauss_jordan_sub(double* S, double* aux, int n_act, const Again& again) {
   GJOrder order;
-  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, order, n_act, GJFromCopy<Ld, kThreads, kSub>{save});
+  const bool singular = gauss_jordan_exchange<Ld, kThreads>(S, aux, order, n_act, again);
   constexpr int kPer = kSub * kSub / kThreads;
   double x[kPer];
 #pragma unroll
@@ -405,7 +417,7 @@ __device__ inline bool sweep_block(double* P, double* aux, int n_act = kBlock) {
     double* Pkr = P + k0 * kPivotLd + r0;
     double* Prk = P + r0 * kPivotLd + k0;
     double* Prr = P + r0 * kPivotLd + r0;
-    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj, U, s == 0 ? kSub : n_act - kSub);
+    singular |= gauss_jordan_sub<kPivotLd, kPivotThreads>(Pkk, gj, s == 0 ? kSub : n_act - kSub, GJFromCopy<kPivotLd, kPivotThreads, kSub>{U});
     small_gemm64(U, kSmallLd, Pkk, kPivotLd, Pkr, kPivotLd, 1.0, false);     // U = P_KK^-1 P_KR
     small_gemm64(Prr, kPivotLd, Prk, kPivotLd, U, kSmallLd, -1.0, true);  // P_RR -= P_RK U
     if (!kSym) small_gemm64(Prk, kPivotLd, Prk, kPivotLd, Pkk, kPivotLd, 1.0, false);  // V = P_RK P_KK^-1
@@ -480,13 +492,13 @@ __global__ void __launch_bounds__(kPivotThreads) sweep_pivot_kernel(double* __re
 
 // Sweep of a single-block matrix whose channels fill at most the leading 64 rows and
 // columns (the rest is identity padding): only the 64x64 block is inverted, in a CTA with
-// 75 KB of shared memory so that two matrices share an SM (its registers hold no third); the padding becomes -I.
-constexpr size_t kPivot64SmemBytes = (size_t(2) * kSub * kSmallLd + kGJAuxDoubles) * sizeof(double);
+// 41 KB of shared memory so that several matrices share an SM; the padding becomes -I.
+constexpr size_t kPivot64SmemBytes = (size_t(kSub) * kSmallLd + kGJAuxDoubles) * sizeof(double);
 template <bool kSym>
 __global__ void __launch_bounds__(kPivotThreads) sweep_pivot64_kernel(double* __restrict__ M, long long mstride, int ld, int n_act, int* status) {
   extern __shared__ double smem[];
   double* S = smem;
-  double* gj = S + 2 * kSub * kSmallLd;
+  double* gj = S + kSub * kSmallLd;
   const int b = blockIdx.x;
   double* Mb = M + (long long)b * mstride;
 #pragma unroll
@@ -495,7 +507,7 @@ __global__ void __launch_bounds__(kPivotThreads) sweep_pivot64_kernel(double* __
     *reinterpret_cast<double2*>(S + (piece >> 5) * kSmallLd + (piece & 31) * 2) = *reinterpret_cast<const double2*>(Mb + (long long)(piece >> 5) * ld + (piece & 31) * 2);
   }
   __syncthreads();
-  const bool singular = gauss_jordan_sub<kSmallLd, kPivotThreads>(S, gj, S + kSub * kSmallLd, n_act);
+  const bool singular = gauss_jordan_sub<kSmallLd, kPivotThreads>(S, gj, n_act, GJFromSource<kSmallLd, kPivotThreads>{Mb, ld});
   if (singular && threadIdx.x == 0) report_status(status, kDeviceSingularPivot, b, 0);
   for (int idx = threadIdx.x; idx < ld * ld; idx += kPivotThreads) {
     const int i = idx / ld, j = idx % ld;
